@@ -24,7 +24,7 @@ EXE = os.path.join(HERE, "kspaceFirstOrder-B200")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-O3",
+CU_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "--compress-mode=size", "-Xcompiler", "-fPIC,-O3",
             "-I" + INCLUDE, "-I" + CSRC]
 CXX_FLAGS = ["-std=c++17", "-O3", "-fPIC", "-I" + INCLUDE, "-I" + CSRC, "-I/usr/local/cuda/include"]
 

@@ -39,8 +39,8 @@ cudaError_t launch_x_r2c(const float* f, float2* S, const Dims& d, const FFTPlan
 cudaError_t launch_x_c2r(const float2* S, float* out, int accumulate, const Dims& d, const FFTPlan& plan,
                          const float2* tw, int L, cudaStream_t st);
 bool tma_col_supported(int n);
-int tma_lines(int n);
-bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n);
+int tma_lines(int n, int v);
+bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n, int v);
 cudaError_t launch_col_tma(bool inv, int n, const ColTmaArgs& a, const float2* tw, cudaStream_t st);
 }  // namespace kwb
 
@@ -77,10 +77,10 @@ void column_pass(const kw_fft3d_plan& p, int axis, bool inv, float2* S, cudaStre
   if (tma_col_supported(n)) {
     ColTmaArgs ca;
     std::memset(&ca, 0, sizeof(ca));
-    if (!make_spec_map(&ca.map[0], S, d, axis, n)) throw std::runtime_error("tensor map of the spectrum");
+    if (!make_spec_map(&ca.map[0], S, d, axis, n, ca.v)) throw std::runtime_error("tensor map of the spectrum");
     ca.nfields = 1;
     ca.dual_field = ca.dual_src = -1;
-    ca.ncx = (d.nxh + tma_lines(n) - 1) / tma_lines(n);
+    ca.ncx = (d.nxh + tma_lines(n, ca.v) - 1) / tma_lines(n, ca.v);
     ca.nouter = axis == 1 ? d.nz : d.ny;
     ca.outer0 = 0;
     ca.yaxis = axis;

@@ -13,140 +13,301 @@
 
 namespace kwb {
 
-// The compile-time plan, chosen so the largest radix sets T = N / RMAX
-// threads per line: 16-point stages first, then 8 / 4 / 2, then 5, 3.
-__host__ __device__ constexpr int ct_stage_count(int n) {
-  if (n <= 0) return -1;
-  int m = n, s = 0;
-  while (m % 16 == 0) { m /= 16; ++s; }
-  const int rs[5] = {8, 4, 2, 5, 3};
-  for (int i = 0; i < 5; ++i)
-    while (m % rs[i] == 0) { m /= rs[i]; ++s; }
-  return m == 1 ? s : -1;
-}
-
-__host__ __device__ constexpr int ct_radix(int n, int stage) {
-  if (n <= 0) return 1;
-  int m = n, s = 0;
-  while (m % 16 == 0) {
-    if (s == stage) return 16;
-    m /= 16;
-    ++s;
-  }
-  const int rs[5] = {8, 4, 2, 5, 3};
-  for (int i = 0; i < 5; ++i)
-    while (m % rs[i] == 0) {
-      if (s == stage) return rs[i];
-      m /= rs[i];
-      ++s;
-    }
-  return 1;
-}
-
-__host__ __device__ constexpr int ct_ns(int n, int stage) {  // product of the radices before `stage`
-  int p = 1;
-  for (int s = 0; s < stage; ++s) p *= ct_radix(n, s);
-  return p;
-}
-
-__host__ __device__ constexpr int ct_rmax(int n) {
-  int r = 1;
-  for (int s = 0; s < ct_stage_count(n); ++s) r = ct_radix(n, s) > r ? ct_radix(n, s) : r;
-  return r;
-}
-
-template <int N>
-struct Ct {
-  static constexpr int S = ct_stage_count(N);
-  static constexpr int RMAX = ct_rmax(N);
-  static constexpr int T = N / RMAX;  // threads per line
-  static_assert(S > 0, "transform length must factor into 2, 3 and 5");
+// ---------------------------------------------------------------------------
+// Radix plans.  A stage costs each thread a read and a write of shared memory
+// per point, two block barriers, the twiddles and the butterflies, so few
+// stages of large, nearly equal radices win (180 = 15 x 12 instead of
+// 4 x 5 x 3 x 3: half the stages, and every thread busy in each).  The plan
+// of a length is found by exhaustive search over its factorisations into the
+// radices there are codelets for, largest first, with the cost model below.
+// Variant 1 is for grids too small to fill the device, where a step is a
+// chain of latencies: the model then counts one thread's own work, so more
+// threads share a line (128 = 8 x 4 x 4 on 16 threads instead of 16 x 8 on 8).
+// ---------------------------------------------------------------------------
+constexpr int kCtMaxStages = 10;
+struct CtPlan {
+  int s;
+  int r[kCtMaxStages];
 };
 
-// Lines per thread block for a compile-time length: about 256 threads, at
-// least 4 lines (a 32-byte sector of complex values per column tile row).
-__host__ __device__ constexpr int ct_lines_of(int n) {
-  if (n <= 0) return 0;
-  int l = 256 / (n / ct_rmax(n));
-  if (l < 4) l = 4;
-  if (l > 32) l = 32;
+__host__ __device__ constexpr int ct_codelet_cost(int r) {  // packed arithmetic instructions, roughly
+  switch (r) {
+    case 2: return 2;
+    case 3: return 8;
+    case 4: return 8;
+    case 5: return 20;
+    case 6: return 22;
+    case 7: return 48;
+    case 8: return 26;
+    case 9: return 62;
+    case 10: return 50;
+    case 12: return 56;
+    case 14: return 110;
+    case 15: return 100;
+    default: return 86;
+  }
+}
+
+// Instructions of one thread per line element it owns (variant 0: block
+// throughput) or in all (variant 1: latency, with 150 for a stage's barriers
+// and shared-memory round trip and 60 per element for the work around the
+// transform), times 1000.  (250 and 40, fewer stages on fewer threads, was
+// slower: 128 x 128 lossless 32 against 25 us per step, 64 x 72 x 80
+// absorbing 124 against 96.)
+__host__ __device__ constexpr long long ct_plan_cost(int n, const CtPlan& p, int variant) {
+  int rmax = 1;
+  for (int i = 0; i < p.s; ++i) rmax = p.r[i] > rmax ? p.r[i] : rmax;
+  const int t = n / rmax;
+  long long c = 0;
+  for (int i = 0; i < p.s; ++i) {
+    const int r = p.r[i], nb = (n / r + t - 1) / t;
+    c += nb * (4 * r + (i ? 6 * (r - 1) : 0) + ct_codelet_cost(r) + 12) + (variant ? 150 : 40);
+  }
+  return variant ? 1000 * (c + 60 * rmax) : 1000 * c / rmax;
+}
+
+__host__ __device__ constexpr void ct_search(int n, int rest, int first, CtPlan& cur, CtPlan& best, long long& cost,
+                                             int variant) {
+  constexpr int radices[13] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  if (rest == 1) {
+    const long long c = ct_plan_cost(n, cur, variant);
+    if (best.s == 0 || c < cost) {
+      best = cur;
+      cost = c;
+    }
+    return;
+  }
+  if (cur.s == kCtMaxStages) return;
+  for (int i = first; i < 13; ++i) {
+    if (rest % radices[i]) continue;
+    cur.r[cur.s++] = radices[i];
+    ct_search(n, rest / radices[i], i, cur, best, cost, variant);
+    --cur.s;
+  }
+}
+
+__host__ __device__ constexpr CtPlan ct_plan(int n, int variant) {
+  CtPlan cur{}, best{};
+  long long cost = 0;
+  if (n > 1) ct_search(n, n, 0, cur, best, cost, variant);
+  return best;
+}
+
+// Ct<N, V>: the plan of length N.  REV (below) runs its stages in the opposite
+// radix order, so that an inverse transform can start from the registers a
+// forward one ends in (CtHandoff).
+template <int N, int V = 0>
+struct Ct {
+  static constexpr CtPlan P = ct_plan(N, V);
+  static constexpr int S = P.s;
+  static_assert(S > 0, "transform length must factor into 2, 3, 5 and 7");
+  static constexpr int rmax() {
+    int r = 1;
+    for (int i = 0; i < P.s; ++i) r = P.r[i] > r ? P.r[i] : r;
+    return r;
+  }
+  static constexpr int RMAX = rmax();
+  static constexpr int T = N / RMAX;  // threads per line
+  static constexpr int held() {       // most elements a thread holds in a stage
+    int h = 0;
+    for (int i = 0; i < P.s; ++i) {
+      const int v = (N / P.r[i] + T - 1) / T * P.r[i];
+      h = v > h ? v : h;
+    }
+    return h;
+  }
+  static constexpr int radix(int stage, bool rev) { return rev ? P.r[S - 1 - stage] : P.r[stage]; }
+  static constexpr int ns(int stage, bool rev) {  // product of the radices before `stage`
+    int p = 1;
+    for (int i = 0; i < stage; ++i) p *= radix(i, rev);
+    return p;
+  }
+};
+
+template <int V>
+struct Ct<0, V> {
+  static constexpr int S = 0, RMAX = 1, T = 1;
+  static constexpr int held() { return 16; }
+};
+
+// ---------------------------------------------------------------------------
+// Tile shapes
+// ---------------------------------------------------------------------------
+// Columns per column tile: rows of 32 to 256 bytes in global memory (a
+// multiple of 4 bins, so a tile's rows are whole 32-byte sectors), 128 to 400
+// threads, and a tile of at most 36 KB.
+__host__ __device__ constexpr int ct_col_lines(int n, int t) {
+  int l = t <= 8 ? 32 : (t <= 20 ? 16 : (t <= 40 ? 8 : 4));
+  while (l > 4 && l * n > 4608) l /= 2;
   return l;
 }
-__host__ __device__ constexpr int ct_threads_of(int n) { return n <= 0 ? 0 : (n / ct_rmax(n)) * ct_lines_of(n); }
 
-template <int N, int STAGE, bool INV, class L>
+// Row pairs per row tile: about 128 threads (variant 1: 64) in as few partly
+// idle warps as possible; an even count where the threads per line are odd
+// (the tile's element count is then even: 16-byte aligned bulk copies).
+__host__ __device__ constexpr int ct_row_lines(int t, int variant) {
+  const int lo = variant ? 32 : 80, hi = variant ? 96 : 160, mid = variant ? 64 : 128;
+  int best = 1, best_score = -1000000;
+  for (int l = 1; l * t <= hi || l == 1; ++l) {
+    if (l * t < lo && (l + 1) * t <= hi) continue;
+    if (l > 1 && (l & 1) && (t & 1)) continue;
+    const int th = l * t, full = (th + 31) / 32 * 32;
+    const int off = th > mid ? th - mid : mid - th;
+    const int score = 1000 * th / full - off;
+    if (score > best_score) {
+      best_score = score;
+      best = l;
+    }
+  }
+  return best;
+}
+
+// Row tile layout: element (l, n) at l * LS + n + n / PAD.  One element of
+// padding per 16 where the first radix is 16 (its outputs, 16 apart, would all
+// fall in one bank), per 32 otherwise; and LS = T mod 16, so the lines that
+// share a warp continue the bank sequence of a line's butterflies.  Over the
+// lengths this gives 1.0-1.6 shared-memory wavefronts per ideal one (the same
+// layout with LS = n + n / 16 + 1: 2 to 6).
+//
+// at(base, l, n0, c, block): the index of element n0 + c given base = (l, n0),
+// c and block compile-time constants once the stage loops are unrolled: base
+// plus a constant where the padding allows it.  block > 0: n0 + c lies in the
+// aligned block of that many elements that n0 lies in.
+template <int N, int V = 0>
+struct CtRow {
+  static constexpr int SH = (N > 0 && Ct<N, V>::RMAX == 16) ? 4 : 5;
+  static constexpr int PAD = 1 << SH;
+  static constexpr int stride() {
+    int ls = N + ((N - 1) >> SH);
+    if (N % 4 == 0 && ls < N + 4) ls = N + 4;  // two raw half-spectrum rows fit one line (RowBulk)
+    while (ls % 16 != Ct<N, V>::T % 16) ++ls;
+    return ls;
+  }
+  static constexpr int LS = stride();
+  __device__ __forceinline__ int operator()(int l, int n) const { return l * LS + n + (n >> SH); }
+  __device__ __forceinline__ int at(int base, int l, int n0, int c, int block) const {
+    if (block > 0 && PAD % block == 0) return base + c;
+    if (c % PAD == 0) return base + c + c / PAD;
+    return (*this)(l, n0 + c);
+  }
+};
+
+// Column tile layout: element (l, n) at n * TL + l.
+template <int TL>
+struct CtCol {
+  __device__ __forceinline__ int operator()(int l, int n) const { return n * TL + l; }
+  __device__ __forceinline__ int at(int base, int, int, int c, int) const { return base + c * TL; }
+};
+
+// ---------------------------------------------------------------------------
+// Stages
+// ---------------------------------------------------------------------------
+// threadIdx.x made opaque to the optimiser: the word it is summed with is 0
+// (tw[0] = exp(0) = 1), but only a shared-memory read at run time tells.  The
+// transforms take the thread's butterfly index from it: without it ptxas
+// hoists every stage's addresses out of a loop over a tile's fields and spills
+// them (k_x_eos at 540 points 132 against 72 registers, k_x_rho at 144 points
+// up to 0.9 KB of spills a thread).  Powers of two keep the plain index: their
+// addresses are base + constant, and recomputing them cost k_x_u and k_x_rho
+// 5 % at 256 points.
+template <int N>
+__device__ __forceinline__ int ct_tid(const float2* tw) {
+  if constexpr ((N & (N - 1)) == 0)
+    return (int)threadIdx.x;
+  else
+    return (int)threadIdx.x + (*reinterpret_cast<const volatile int*>(tw) - 0x3f800000);
+}
+
+// Butterflies per thread in a stage.
+template <int N, int V, int STAGE, bool REV>
+struct CtStage {
+  static constexpr int R = Ct<N, V>::radix(STAGE, REV);
+  static constexpr int NS = Ct<N, V>::ns(STAGE, REV);
+  static constexpr int NR = N / R;
+  static constexpr int T = Ct<N, V>::T;
+  static constexpr int NB = (NR + T - 1) / T;
+  static constexpr int TWS = N / (NS * R);
+  static __device__ __forceinline__ bool has(int j) { return NR % T == 0 || j < NR; }
+};
+
+// Twiddles and butterfly j of a stage.
+template <class G, bool INV>
+__device__ __forceinline__ void ct_butterfly(float2 (&v)[G::R], const float2* __restrict__ tw, int j) {
+  if constexpr (G::NS > 1) {
+    const int step = (j % G::NS) * G::TWS;
+#pragma unroll
+    for (int r = 1; r < G::R; ++r) {
+      float2 w = tw[step * r];
+      if (INV) w.y = -w.y;
+      v[r] = c_mul(v[r], w);
+    }
+  }
+  dft<G::R, INV>(v);
+}
+
+// Inputs of a thread's butterflies from `buf`.
+template <class G, class L>
+__device__ __forceinline__ void ct_load(float2 (&v)[G::R], const float2* buf, int l, int j, L lay) {
+  const int base = lay(l, j);
+#pragma unroll
+  for (int r = 0; r < G::R; ++r) v[r] = buf[lay.at(base, l, j, r * G::NR, 0)];
+}
+
+// Outputs of butterfly j to `buf`.
+template <class G, class L>
+__device__ __forceinline__ void ct_store(const float2 (&v)[G::R], float2* buf, int l, int j, L lay) {
+  const int idx = (j / G::NS) * (G::NS * G::R) + j % G::NS;
+  const int base = lay(l, idx);
+#pragma unroll
+  for (int r = 0; r < G::R; ++r) buf[lay.at(base, l, idx, r * G::NS, G::NS * G::R)] = v[r];
+}
+
+// One in-place stage: inputs to registers, barrier, outputs, barrier.
+template <int N, int V, int STAGE, bool INV, bool REV, class L>
 __device__ __forceinline__ void ct_stage(float2* buf, const float2* __restrict__ tw, int l, int tid, L lay) {
-  constexpr int R = ct_radix(N, STAGE);
-  constexpr int NS = ct_ns(N, STAGE);
-  constexpr int NR = N / R;
-  constexpr int T = Ct<N>::T;
-  constexpr int NB = (NR + T - 1) / T;
-  constexpr int TWS = N / (NS * R);
-  float2 v[NB][R];
+  using G = CtStage<N, V, STAGE, REV>;
+  float2 v[G::NB][G::R];
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const int j = tid + i * T;
-    if (NR % T == 0 || j < NR) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[i][r] = buf[lay(l, j + r * NR)];
-      if constexpr (NS > 1) {
-        const int k = j % NS;
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          float2 w = tw[k * r * TWS];
-          if (INV) w.y = -w.y;
-          v[i][r] = c_mul(v[i][r], w);
-        }
-      }
-      dft<R, INV>(v[i]);
+  for (int i = 0; i < G::NB; ++i) {
+    const int j = tid + i * G::T;
+    if (G::has(j)) {
+      ct_load<G>(v[i], buf, l, j, lay);
+      ct_butterfly<G, INV>(v[i], tw, j);
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const int j = tid + i * T;
-    if (NR % T == 0 || j < NR) {
-      const int k = j % NS;
-      const int idx = (j / NS) * NS * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) buf[lay(l, idx + r * NS)] = v[i][r];
-    }
+  for (int i = 0; i < G::NB; ++i) {
+    const int j = tid + i * G::T;
+    if (G::has(j)) ct_store<G>(v[i], buf, l, j, lay);
   }
   __syncthreads();
 }
 
-// One stage with caller-supplied element access: ld(l, pos) returns the
-// input element, st(l, pos, v) stores an output element.  No barriers: the
-// caller synchronises (between the loads and stores when they alias, and
-// before the outputs are read).
-template <int N, int STAGE, bool INV, class LD, class ST>
-__device__ __forceinline__ void ct_stage_io(const float2* __restrict__ tw, int l, int tid, LD ld, ST st) {
-  constexpr int R = ct_radix(N, STAGE);
-  constexpr int NS = ct_ns(N, STAGE);
-  constexpr int NR = N / R;
-  constexpr int T = Ct<N>::T;
-  constexpr int NB = (NR + T - 1) / T;
-  constexpr int TWS = N / (NS * R);
+// Stages FIRST .. LAST - 1.
+template <int N, int V, int FIRST, int LAST, bool INV, bool REV, class L>
+__device__ __forceinline__ void ct_stages(float2* buf, const float2* __restrict__ tw, int l, int tid, L lay) {
+  if constexpr (FIRST < LAST) {
+    ct_stage<N, V, FIRST, INV, REV>(buf, tw, l, tid, lay);
+    ct_stages<N, V, FIRST + 1, LAST, INV, REV>(buf, tw, l, tid, lay);
+  }
+}
+
+// The last stage with a caller-supplied output: st(pos, v) receives element
+// pos of this thread's line.  No barriers.
+template <int N, int V, bool INV, bool REV, class L, class ST>
+__device__ __forceinline__ void ct_last_st(const float2* buf, const float2* __restrict__ tw, int l, int tid, L lay,
+                                           ST st) {
+  using G = CtStage<N, V, Ct<N, V>::S - 1, REV>;
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const int j = tid + i * T;
-    if (NR % T == 0 || j < NR) {
-      float2 v[R];
+  for (int i = 0; i < G::NB; ++i) {
+    const int j = tid + i * G::T;
+    if (G::has(j)) {
+      float2 v[G::R];
+      ct_load<G>(v, buf, l, j, lay);
+      ct_butterfly<G, INV>(v, tw, j);
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = ld(l, j + r * NR);
-      const int k = j % NS;
-      if constexpr (NS > 1) {
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-          float2 w = tw[k * r * TWS];
-          if (INV) w.y = -w.y;
-          v[r] = c_mul(v[r], w);
-        }
-      }
-      dft<R, INV>(v);
-      const int idx = (j / NS) * NS * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) st(l, idx + r * NS, v[r]);
+      for (int r = 0; r < G::R; ++r) st(j + r * G::NS, v[r]);  // j < NS in the last stage
     }
   }
 }
@@ -156,103 +317,62 @@ __device__ __forceinline__ void ct_stage_io(const float2* __restrict__ tw, int l
 // build each packed line from two raw half-spectrum rows on the fly).  In
 // place like ct_stage: every input is loaded before the block barrier and
 // every output stored after it, so the inputs may alias the output buffer.
-template <int N, bool INV, class L, class LD>
+template <int N, int V, bool INV, class L, class LD>
 __device__ __forceinline__ void ct_stage0_ld(float2* buf, int l, int tid, L lay, LD ld) {
-  constexpr int R = ct_radix(N, 0);
-  constexpr int NR = N / R;
-  constexpr int T = Ct<N>::T;
-  constexpr int NB = (NR + T - 1) / T;
-  float2 v[NB][R];
+  using G = CtStage<N, V, 0, false>;
+  float2 v[G::NB][G::R];
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const int j = tid + i * T;
-    if (NR % T == 0 || j < NR) {
+  for (int i = 0; i < G::NB; ++i) {
+    const int j = tid + i * G::T;
+    if (G::has(j)) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[i][r] = ld(l, j + r * NR);
-      dft<R, INV>(v[i]);  // first stage: no twiddles
+      for (int r = 0; r < G::R; ++r) v[i][r] = ld(l, j + r * G::NR);
+      ct_butterfly<G, INV>(v[i], nullptr, j);  // first stage: no twiddles
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const int j = tid + i * T;
-    if (NR % T == 0 || j < NR) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) buf[lay(l, j * R + r)] = v[i][r];
-    }
+  for (int i = 0; i < G::NB; ++i) {
+    const int j = tid + i * G::T;
+    if (G::has(j)) ct_store<G>(v[i], buf, l, j, lay);
   }
   __syncthreads();
-}
-
-template <int N, int STAGE, bool INV, class L>
-__device__ __forceinline__ void ct_stages(float2* buf, const float2* __restrict__ tw, int l, int tid, L lay) {
-  if constexpr (STAGE < Ct<N>::S) {
-    ct_stage<N, STAGE, INV>(buf, tw, l, tid, lay);
-    ct_stages<N, STAGE + 1, INV>(buf, tw, l, tid, lay);
-  }
 }
 
 // Register hand-off between a forward transform and an inverse one of the
-// same line.  Thread `tid` of a line owns positions tid + T*m, m < N/T, in
-// two places: they are the outputs of its butterflies in the last stage
-// (position j + r*NS, NS = N / R_last, j = tid + i*T) and the inputs of its
-// butterflies in the first stage (position j + r*N/R_0), provided T divides
-// N / R_last and N / R_0 (the largest radix is a multiple of the first and
-// last ones: 64 = 16*4, 128 = 16*8, 256 = 16*16).  A spectral operator can
-// then be applied in registers between the forward transform's last stage
-// and the inverse transform's first, without a shared-memory round trip.
-template <int N>
+// same line.  The forward transform runs its stages in the opposite radix
+// order (REV), so its last stage has the largest radix, one butterfly per
+// thread, and leaves butterfly tid's outputs at positions tid + T m, m <
+// RMAX; the inverse transform's first stage has the same radix and its
+// butterfly tid reads exactly those positions.  So the thread that ends the
+// one starts the other, and a spectral operator is applied in between in
+// registers with no shared-memory pass, for every length.
+template <int N, int V>
 struct CtHandoff {
-  static constexpr int S = Ct<N>::S;
-  static constexpr int T = Ct<N>::T;
-  static constexpr int M = N / T;  // positions per thread
-  static constexpr bool OK = S >= 2 && (ct_ns(N, S - 1) % T == 0) && ((N / ct_radix(N, 0)) % T == 0);
+  using G = CtStage<N, V, Ct<N, V>::S - 1, true>;  // forward, last stage
+  using H = CtStage<N, V, 0, false>;               // inverse, first stage
+  static constexpr int M = Ct<N, V>::RMAX;         // positions per thread
+  static_assert(Ct<N, V>::S >= 2 && G::NB == 1 && H::NB == 1 && G::R == M && H::R == M && G::NS == Ct<N, V>::T &&
+                    H::NR == Ct<N, V>::T,
+                "the last and first stages face each other");
 };
 
-// Forward last stage of line `l` read from `src`; u[m] receives position tid + T*m.
-template <int N, class L>
+// Forward last stage of line `l` read from `src`; u[m] receives position tid + T m.
+template <int N, int V, class L>
 __device__ __forceinline__ void ct_fwd_last_to_regs(const float2* __restrict__ src, const float2* __restrict__ tw,
-                                                    int l, int tid, L lay, float2 (&u)[CtHandoff<N>::M]) {
-  static_assert(CtHandoff<N>::OK, "no register hand-off for this plan");
-  constexpr int STAGE = Ct<N>::S - 1;
-  constexpr int R = ct_radix(N, STAGE);
-  constexpr int NS = ct_ns(N, STAGE);  // = N / R: the stride of the outputs
-  constexpr int NR = N / R;
-  constexpr int T = Ct<N>::T;
-  constexpr int TWS = N / (NS * R);
-#pragma unroll
-  for (int i = 0; i < NR / T; ++i) {
-    const int j = tid + i * T;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[lay(l, j + r * NR)];
-#pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = c_mul(v[r], tw[j * r * TWS]);  // k = j % NS = j
-    dft<R, false>(v);
-#pragma unroll
-    for (int r = 0; r < R; ++r) u[i + r * (NS / T)] = v[r];  // position j + r * NS
-  }
+                                                    int l, int tid, L lay, float2 (&u)[CtHandoff<N, V>::M]) {
+  using G = typename CtHandoff<N, V>::G;
+  ct_load<G>(u, src, l, tid, lay);
+  ct_butterfly<G, false>(u, tw, tid);
 }
 
-// Inverse first stage from registers (u[m] = position tid + T*m); stores its
-// outputs to `dst` in the order the next stage reads (as ct_stage does).
-template <int N, class L>
-__device__ __forceinline__ void ct_inv_first_from_regs(const float2 (&u)[CtHandoff<N>::M], float2* __restrict__ dst,
+// Inverse first stage from u; stores its outputs to `dst` for the next stage.
+template <int N, int V, class L>
+__device__ __forceinline__ void ct_inv_first_from_regs(float2 (&u)[CtHandoff<N, V>::M], float2* __restrict__ dst,
                                                        int l, int tid, L lay) {
-  static_assert(CtHandoff<N>::OK, "no register hand-off for this plan");
-  constexpr int R = ct_radix(N, 0);
-  constexpr int NR = N / R;
-  constexpr int T = Ct<N>::T;
-#pragma unroll
-  for (int i = 0; i < NR / T; ++i) {
-    const int j = tid + i * T;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = u[i + r * (NR / T)];  // position j + r * NR
-    dft<R, true>(v);
-#pragma unroll
-    for (int r = 0; r < R; ++r) dst[lay(l, j * R + r)] = v[r];
-  }
+  using H = typename CtHandoff<N, V>::H;
+  ct_butterfly<H, true>(u, nullptr, tid);
+  ct_store<H>(u, dst, l, tid, lay);
 }
 
 // In-place transform of LINES lines by T * LINES threads.  LINE_FAST maps
@@ -260,28 +380,24 @@ __device__ __forceinline__ void ct_inv_first_from_regs(const float2 (&u)[CtHando
 // adjacent in shared memory); otherwise to consecutive butterflies of one
 // line (row tiles).  Must be called by every thread of the block (it
 // synchronises); the caller synchronises before the call.
-template <int N, bool INV, bool LINE_FAST, int LINES, class L>
+template <int N, int V, bool INV, bool LINE_FAST, int LINES, class L>
 __device__ __forceinline__ void ct_fft(float2* buf, const float2* __restrict__ tw, L lay) {
-  constexpr int T = Ct<N>::T;
-  int l, tid;
-  if (LINE_FAST) {
-    l = threadIdx.x % LINES;
-    tid = threadIdx.x / LINES;
-  } else {
-    l = threadIdx.x / T;
-    tid = threadIdx.x - l * T;
-  }
-  ct_stages<N, 0, INV>(buf, tw, l, tid, lay);
+  constexpr int T = Ct<N, V>::T;
+  const int id = ct_tid<N>(tw);
+  const int l = LINE_FAST ? id % LINES : id / T;
+  const int tid = LINE_FAST ? id / LINES : id - l * T;
+  ct_stages<N, V, 0, Ct<N, V>::S, INV, false>(buf, tw, l, tid, lay);
 }
 
 // Row tiles (consecutive threads on consecutive butterflies of a line): the
 // first stage reads its inputs through `ld`, the others run in place.
-template <int N, bool INV, class L, class LD>
+template <int N, int V, bool INV, class L, class LD>
 __device__ __forceinline__ void ct_fft_rows_ld(float2* buf, const float2* __restrict__ tw, L lay, LD ld) {
-  constexpr int T = Ct<N>::T;
-  const int l = threadIdx.x / T, tid = threadIdx.x - l * T;
-  ct_stage0_ld<N, INV>(buf, l, tid, lay, ld);
-  ct_stages<N, 1, INV>(buf, tw, l, tid, lay);
+  constexpr int T = Ct<N, V>::T;
+  const int id = ct_tid<N>(tw);
+  const int l = id / T, tid = id - l * T;
+  ct_stage0_ld<N, V, INV>(buf, l, tid, lay, ld);
+  ct_stages<N, V, 1, Ct<N, V>::S, INV, false>(buf, tw, l, tid, lay);
 }
 
 }  // namespace kwb

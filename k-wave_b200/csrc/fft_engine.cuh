@@ -187,15 +187,87 @@ __device__ __forceinline__ void dft16(float2* v) {
   }
   dft8<INV>(e);
   dft8<INV>(o);
-  // W16^k = exp(-+ i k pi / 8)
+  // W16^k = exp(-+ i k pi / 8); k = 0 is 1, k = 4 a quarter turn, k = 2 and 6 diagonals
   const float wc[8] = {1.f, c1, r, s1, 0.f, -s1, -r, -c1};
   const float ws[8] = {0.f, s1, r, c1, 1.f, c1, r, s1};
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    float2 w = make_float2(wc[k], INV ? ws[k] : -ws[k]);
-    float2 t = c_mul(o[k], w);
+    float2 t;
+    if (k == 0) {
+      t = o[k];
+    } else if (k == 4) {
+      t = c_rot<INV>(o[k]);
+    } else if (k == 2) {
+      t = INV ? make_float2(r * (o[k].x - o[k].y), r * (o[k].x + o[k].y))
+              : make_float2(r * (o[k].x + o[k].y), r * (o[k].y - o[k].x));
+    } else if (k == 6) {
+      t = INV ? make_float2(-r * (o[k].x + o[k].y), r * (o[k].x - o[k].y))
+              : make_float2(r * (o[k].y - o[k].x), -r * (o[k].x + o[k].y));
+    } else {
+      t = c_mul(o[k], make_float2(wc[k], INV ? ws[k] : -ws[k]));
+    }
     v[k] = c_add(e[k], t);
     v[k + 8] = c_sub(e[k], t);
+  }
+}
+
+template <int R, bool INV>
+__device__ __forceinline__ void dft(float2* v);
+
+// R = A B with A and B coprime (6, 10, 12, 14, 15): the prime-factor form
+// (Good 1958), A-point and B-point transforms with no twiddles between them.
+// Input n = (B n1 + A n2) mod R; output k = (B b k1 + A a k2) mod R with
+// b = B^-1 mod A and a = A^-1 mod B.
+__host__ __device__ constexpr int inv_mod(int x, int m) {
+  for (int i = 1; i < m; ++i)
+    if (x % m * i % m == 1) return i;
+  return 1;
+}
+template <int A, int B, bool INV>
+__device__ __forceinline__ void dft_pfa(float2* v) {
+  constexpr int R = A * B, eb = B * inv_mod(B, A), ea = A * inv_mod(A, B);
+  float2 t[B][A];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) {
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) t[n2][n1] = v[(B * n1 + A * n2) % R];
+    dft<A, INV>(t[n2]);
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    float2 b[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) b[n2] = t[n2][k1];
+    dft<B, INV>(b);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) v[(eb * k1 + ea * k2) % R] = b[k2];
+  }
+}
+
+// 9-point: 3 x 3 with W9^(n2 k1) between the two layers.
+template <bool INV>
+__device__ __forceinline__ void dft9(float2* v) {
+  // cos / sin of 2 pi k / 9, k = 1, 2, 4
+  const float c[3] = {0.766044443118978035f, 0.173648177666930349f, -0.939692620785908384f};
+  const float s[3] = {0.642787609686539326f, 0.984807753012208059f, 0.342020143325668733f};
+  float2 t[3][3];
+#pragma unroll
+  for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+    for (int n1 = 0; n1 < 3; ++n1) t[n2][n1] = v[3 * n1 + n2];
+    dft3<INV>(t[n2]);
+  }
+  auto w = [&](float2 a, int i) { return c_mul(a, make_float2(c[i], INV ? s[i] : -s[i])); };
+  t[1][1] = w(t[1][1], 0);
+  t[1][2] = w(t[1][2], 1);
+  t[2][1] = w(t[2][1], 1);
+  t[2][2] = w(t[2][2], 2);
+#pragma unroll
+  for (int k1 = 0; k1 < 3; ++k1) {
+    float2 b[3] = {t[0][k1], t[1][k1], t[2][k1]};
+    dft3<INV>(b);
+#pragma unroll
+    for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = b[k2];
   }
 }
 
@@ -213,6 +285,18 @@ __device__ __forceinline__ void dft(float2* v) {
     dft7<INV>(v);
   } else if constexpr (R == 8) {
     dft8<INV>(v);
+  } else if constexpr (R == 9) {
+    dft9<INV>(v);
+  } else if constexpr (R == 6) {
+    dft_pfa<2, 3, INV>(v);
+  } else if constexpr (R == 10) {
+    dft_pfa<2, 5, INV>(v);
+  } else if constexpr (R == 12) {
+    dft_pfa<4, 3, INV>(v);
+  } else if constexpr (R == 14) {
+    dft_pfa<2, 7, INV>(v);
+  } else if constexpr (R == 15) {
+    dft_pfa<3, 5, INV>(v);
   } else if constexpr (R == 16) {
     dft16<INV>(v);
   }

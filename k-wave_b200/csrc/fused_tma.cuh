@@ -16,22 +16,18 @@ namespace kwb {
 
 int tma_num_sms();  // multiprocessors of the current device
 
-// Lines per TMA tile: the compile-time tile's line count rounded down to an
-// even number, so every tile starts at a bin index x = cx * LINES whose byte
-// offset (8-byte bins) is a multiple of 16, as tensor copies require.
-__host__ __device__ constexpr int tma_lines_of(int n) {
-  return ct_lines_of(n) & ~1;  // ct_lines_of is at least 4
-}
-
-template <int NC>
+// Lines per TMA tile: the column tile's, a multiple of 4, so every tile starts
+// at a bin index x = cx * LINES whose byte offset (8-byte bins) is a multiple
+// of 32 (tensor copies require 16).
+template <int NC, int V>
 struct TTile {
-  static constexpr int LINES = tma_lines_of(NC);
-  static constexpr int THREADS = Ct<NC>::T * LINES;
+  static constexpr int LINES = ct_col_lines(NC, Ct<NC, V>::T);
+  static constexpr int THREADS = Ct<NC, V>::T * LINES;
   static constexpr int ELEMS = LINES * NC;
   static constexpr unsigned BYTES = ELEMS * sizeof(float2);
   // Stage stride in elements: tensor copies read and write shared memory at
   // 128-byte aligned addresses, so each stage is padded to a multiple of 128
-  // bytes (a tile of 14 lines of 90 points is 10080 bytes).
+  // bytes.
   static constexpr int STRIDE = (int)((BYTES + 127u) / 128u * 128u / sizeof(float2));
 };
 
@@ -50,36 +46,34 @@ __device__ __forceinline__ void tile_coords(int yaxis, int cx, int o, int lines,
 // only that operator's arithmetic in the kernel body.
 enum FusedClass { FC_GRAD = 0, FC_NABLA = 1, FC_SRCK = 2 };
 
-// Blocks per SM the register budget is sized for: three for the hand-off
-// lengths' single-output pass, two otherwise.
-template <int NC, int MODE>
+// Blocks per SM the register budget is sized for: about 768 threads for the
+// single-output pass, 512 otherwise and where a stage holds more than 16
+// elements a thread (180 = 15 x 12 spilled 0.26 KB a thread at 768).
+template <int NC, int V, int MODE>
 struct FusedBounds {
-  static constexpr int MIN_BLOCKS = (MODE && CtHandoff<NC>::OK && Ct<NC>::S == 2) ? 3 : 2;
+  static constexpr int TH = TTile<NC, V>::THREADS;
+  static constexpr int WANT = MODE && Ct<NC, V>::held() <= 16 ? 768 : 512;
+  static constexpr int MIN_BLOCKS = WANT / TH > 0 ? WANT / TH : 1;
 };
 
 // MODE 1: every input has a single output (in place in the input stage: two
 // tile buffers, three blocks per SM).
 // MODE 0: the forward transform is kept and each output multiplied from it
 // into a third buffer (two blocks per SM).
-// For the two-stage lengths 64, 128 and 256 the operator is applied in
-// registers between the forward transform's last stage and the inverse's
-// first (CtHandoff) and the inverse's last stage writes the output; for the
-// other lengths the forward transform, the operator and the inverse each
-// pass through shared memory and the output is stored from there.  (The
-// gradient's pair of outputs, kappa and kappa times the transform axis'
-// derivative, also fits the in-place form with both taken from the hand-off
-// registers, but at three blocks per SM that spills and measured slower:
-// 1.338 against 1.330 ms.)
-template <int NC, int CLS, int MODE>
-__global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN_BLOCKS) k_fused_tma(const __grid_constant__ FusedTmaArgs a,
+// The operator is applied in registers between the forward transform's last
+// stage and the inverse's first (CtHandoff), and the inverse's last stage
+// writes the output.  (The gradient's pair of outputs, kappa and kappa times
+// the transform axis' derivative, also fits the in-place form with both taken
+// from the hand-off registers, but at three blocks per SM that spills and
+// measured slower at 256 points: 1.338 against 1.330 ms per 256^3 step.)
+template <int NC, int V, int CLS, int MODE>
+__global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE>::MIN_BLOCKS) k_fused_tma(const __grid_constant__ FusedTmaArgs a,
                                                                      const float2* __restrict__ tw_g,
                                                                      const __grid_constant__ SpecTables T) {
-  constexpr int TL = TTile<NC>::LINES;
-  constexpr int E = TTile<NC>::STRIDE;  // stage stride (the tile, padded to 128 bytes)
-  constexpr int TH = TTile<NC>::THREADS;
-  // register hand-off between the transforms (two-stage plans: the forward's
-  // first stage, then its last; the inverse's first, then its last)
-  constexpr bool HO = CtHandoff<NC>::OK && Ct<NC>::S == 2;
+  constexpr int TL = TTile<NC, V>::LINES;
+  constexpr int E = TTile<NC, V>::STRIDE;  // stage stride (the tile, padded to 128 bytes)
+  constexpr int TH = TTile<NC, V>::THREADS;
+  constexpr int S = Ct<NC, V>::S;
   extern __shared__ __align__(128) unsigned char smraw[];
   float2* inb = reinterpret_cast<float2*>(smraw);  // 2 input stages
   float2* W = MODE ? nullptr : inb + 2 * E;        // product / inverse-transform buffer (MODE 0)
@@ -128,7 +122,7 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
     const int s = j & 1;
     int g, cx, o, x, y, z;
     decode(t, g, cx, o);
-    mbar_expect_tx(&bar[s], TTile<NC>::BYTES);  // a remainder box holds as many bytes
+    mbar_expect_tx(&bar[s], TTile<NC, V>::BYTES);  // a remainder box holds as many bytes
     if (t == a.wait.skip_tile) return;  // test hook: announced, never issued
     if (cx >= 0) {
       tile_coords(a.yaxis, cx, o, TL, x, y, z);
@@ -145,13 +139,13 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
     if (blockIdx.x < ntiles) issue(blockIdx.x, 0);
     if (blockIdx.x + gridDim.x < ntiles) issue(blockIdx.x + gridDim.x, 1);
   }
-  const ColLayout lay{TL};
+  const CtCol<TL> lay{};
   // the line mapping fixes this thread's column (kx) for every pass
   const int l = threadIdx.x % TL, tid = threadIdx.x / TL;
   const float cdt2sq = T.cdt2 * T.cdt2;
   constexpr int TPL = TH / TL;  // threads per line
-  constexpr int M = CtHandoff<NC>::M;
-  static_assert(TPL == Ct<NC>::T, "one line per group of T threads");
+  constexpr int M = CtHandoff<NC, V>::M;
+  static_assert(TPL == Ct<NC, V>::T, "one line per group of T threads");
   bool aborted = false;
   int it = 0;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
@@ -238,35 +232,15 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
         dst2 += loff;
         dsc = __ldg(a.dual_tab[g * a.fanout + q] + ol);
       }
-      auto ld_w = [&](int ll, int pos) -> float2 { return src[lay(ll, pos)]; };
-      auto st_g = [&](int, int pos, float2 v) {  // (the line is this thread's, folded into loff)
+      auto st_g = [&](int pos, float2 v) {  // (the line is this thread's, folded into loff)
         if (valid) {
           dst[pos * a.lstride] = v;
           if (dst2) dst2[pos * a.lstride] = c_mul(v, dsc);
         }
       };
-      if constexpr (HO) ct_stage_io<NC, 1, true>(tw, l, tid, ld_w, st_g);  // stage 1 is the last
+      ct_last_st<NC, V, true, false>(src, tw, l, tid, lay, st_g);
       fence_async_smem();  // the reads of src come before a TMA refill of it
       __syncthreads();     // src is reused by the next inverse
-    };
-    // every position of the thread's line, from src to the output (no hand-off)
-    auto store_all = [&](int q, const float2* src) {
-      float2* dst = a.outp[g * a.fanout + q] + loff;
-      float2* dst2 = a.dual_outp[g * a.fanout + q];
-      float2 dsc = make_float2(0.f, 0.f);
-      if (dst2) {
-        dst2 += loff;
-        dsc = __ldg(a.dual_tab[g * a.fanout + q] + ol);
-      }
-      if (valid) {
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const int pos = tid + TPL * m;
-          const float2 v = src[lay(l, pos)];
-          dst[pos * a.lstride] = v;
-          if (dst2) dst2[pos * a.lstride] = c_mul(v, dsc);
-        }
-      }
     };
     auto refill = [&]() {  // F is consumed: refill this input stage with the tile two ahead
       if (threadIdx.x == 0) {
@@ -280,41 +254,27 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
       break;
     }
     if (threadIdx.x == 0) inflight &= ~(1u << s);
-    if constexpr (MODE == 1 && !HO) {
-      ct_fft<NC, false, true, TL>(F, tw, lay);
-      {
-        float2 u[M];
-#pragma unroll
-        for (int m = 0; m < M; ++m) u[m] = F[lay(l, tid + TPL * m)];
-        apply(setup(0), u);
-#pragma unroll
-        for (int m = 0; m < M; ++m) F[lay(l, tid + TPL * m)] = u[m];  // this thread's own positions
-      }
-      __syncthreads();
-      ct_fft<NC, true, true, TL>(F, tw, lay);
-      store_all(0, F);
-      fence_async_smem();  // the reads of F come before its TMA refill
-      __syncthreads();
-      refill();
-    } else if constexpr (MODE == 1) {
-      float2 u[M];
-      // forward first stage in place; last stage, operator and inverse first
-      // stage in registers, the latter's outputs back into F once every
-      // thread has read its inputs; inverse last stage to the output; then F
-      // takes the tile two ahead
-      ct_stage<NC, 0, false>(F, tw, l, tid, lay);
-      ct_fwd_last_to_regs<NC>(F, tw, l, tid, lay, u);
+    float2 u[M];
+    ct_stages<NC, V, 0, S - 1, false, true>(F, tw, l, tid, lay);
+    ct_fwd_last_to_regs<NC, V>(F, tw, l, tid, lay, u);
+    if constexpr (MODE == 1) {
+      // operator and inverse first stage in registers, the latter's outputs
+      // back into F once every thread has read its inputs; inverse last
+      // stage to the output; then F takes the tile two ahead
       apply(setup(0), u);
       __syncthreads();
-      ct_inv_first_from_regs<NC>(u, F, l, tid, lay);
+      ct_inv_first_from_regs<NC, V>(u, F, l, tid, lay);
       __syncthreads();
+      ct_stages<NC, V, 1, S - 1, true, false>(F, tw, l, tid, lay);
       finish(0, F);
       refill();
     } else {
-      // several outputs of one input: the forward transform stays in F; each
-      // output is read from it in the hand-off order, multiplied in registers
-      // and given the inverse first stage on the way to W
-      ct_fft<NC, false, true, TL>(F, tw, lay);
+      // several outputs of one input: the forward transform is kept in F, each
+      // thread's own positions; each output is read from it, multiplied in
+      // registers and given the inverse first stage on the way to W
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < M; ++m) F[lay(l, tid + TPL * m)] = u[m];
       // a first output of kappa alone (the gradient pass: kappa P, then kappa
       // P times the axis derivative) leaves kappa * scale * F in F, so the
       // later outputs carrying kappa skip its evaluation (c_mul by 1 + 0i is
@@ -322,7 +282,6 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
       bool kf = false;
 #pragma unroll 1
       for (int q = 0; q < a.fanout; ++q) {
-        float2 u[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) u[m] = F[lay(l, tid + TPL * m)];
         const OpEval ev = setup(q);
@@ -334,22 +293,12 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
             kf = true;
           }
         }
-        if constexpr (HO) {
-          ct_inv_first_from_regs<NC>(u, W, l, tid, lay);
-        } else {
-#pragma unroll
-          for (int m = 0; m < M; ++m) W[lay(l, tid + TPL * m)] = u[m];
-        }
+        ct_inv_first_from_regs<NC, V>(u, W, l, tid, lay);
         if (q + 1 == a.fanout) fence_async_smem();
         __syncthreads();
         if (q + 1 == a.fanout) refill();
-        if constexpr (HO) {
-          finish(q, W);
-        } else {
-          ct_fft<NC, true, true, TL>(W, tw, lay);
-          store_all(q, W);
-          __syncthreads();  // W is rewritten by the next output
-        }
+        ct_stages<NC, V, 1, S - 1, true, false>(W, tw, l, tid, lay);
+        finish(q, W);
       }
     }
   }
@@ -358,33 +307,38 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS, FusedBounds<NC, MODE>::MIN
       if (inflight & (1u << s)) mbar_wait(&bar[s], (parity_bits >> s) & 1, nullptr, a.wait.limit_ns);
 }
 
-template <int NC, int CLS, int MODE>
+template <int NC, int V, int CLS, int MODE>
 cudaError_t fused_tma_t(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st) {
-  const size_t sm = (MODE ? 2 : 3) * TTile<NC>::STRIDE * sizeof(float2) + NC * sizeof(float2) + 2 * sizeof(uint64_t) +
+  const size_t sm = (MODE ? 2 : 3) * TTile<NC, V>::STRIDE * sizeof(float2) + NC * sizeof(float2) + 2 * sizeof(uint64_t) +
                     3 * NC * sizeof(float2) + NC * sizeof(float);
-  auto k = k_fused_tma<NC, CLS, MODE>;
+  auto k = k_fused_tma<NC, V, CLS, MODE>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TTile<NC>::THREADS, sm);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TTile<NC, V>::THREADS, sm);
   const int ntiles = a.nin * (a.ncx * a.nouter + a.nrem);
   const int grid = std::min(ntiles, std::max(1, per_sm) * tma_num_sms());
-  const cudaError_t e = launch_pdl(k, dim3(grid), dim3(TTile<NC>::THREADS), sm, st, a, tw, T);
+  const cudaError_t e = launch_pdl(k, dim3(grid), dim3(TTile<NC, V>::THREADS), sm, st, a, tw, T);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// The fused last-axis pass of one length, dispatched on the operator class
-// (MODE 0, several outputs per input, only for the gradient class).
-template <int NC>
-cudaError_t fused_tma_cls(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st) {
+// The fused last-axis pass of one length, dispatched on the plan variant and
+// the operator class (MODE 0, several outputs per input, only for the
+// gradient class).
+template <int NC, int V>
+cudaError_t fused_tma_v(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st) {
   const int kind = a.op[0].kind;
   const bool one = a.fanout == 1;
   if (kind == OP_GRAD_POS || kind == OP_GRAD_NEG || kind == OP_KAPPA || kind == OP_SHIFT_NEG ||
       kind == OP_KAPPA_SHIFT_NEG) {
-    return one ? fused_tma_t<NC, FC_GRAD, 1>(a, tw, T, st) : fused_tma_t<NC, FC_GRAD, 0>(a, tw, T, st);
+    return one ? fused_tma_t<NC, V, FC_GRAD, 1>(a, tw, T, st) : fused_tma_t<NC, V, FC_GRAD, 0>(a, tw, T, st);
   }
   if (!one) return cudaErrorInvalidValue;
-  if (kind == OP_NABLA1 || kind == OP_NABLA2) return fused_tma_t<NC, FC_NABLA, 1>(a, tw, T, st);
-  return fused_tma_t<NC, FC_SRCK, 1>(a, tw, T, st);
+  if (kind == OP_NABLA1 || kind == OP_NABLA2) return fused_tma_t<NC, V, FC_NABLA, 1>(a, tw, T, st);
+  return fused_tma_t<NC, V, FC_SRCK, 1>(a, tw, T, st);
+}
+template <int NC>
+cudaError_t fused_tma_cls(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st) {
+  return a.v ? fused_tma_v<NC, 1>(a, tw, T, st) : fused_tma_v<NC, 0>(a, tw, T, st);
 }
 
 #define KWB_FUSED_EXTERN(N) \

@@ -115,11 +115,12 @@ struct CtEntry {
   decltype(&CtKernels<0>::x_eos) x_eos;
   decltype(&CtKernels<0>::x_r2c) x_r2c;
   decltype(&CtKernels<0>::x_c2r) x_c2r;
+  decltype(&CtKernels<0>::threads_per_line) threads_per_line;
 };
 
 #define KWB_ENTRY(N)                                                                                  \
   {N, &CtKernels<N>::col_fft, &CtKernels<N>::fused, &CtKernels<N>::x_u, &CtKernels<N>::x_rho,          \
-   &CtKernels<N>::x_eos, &CtKernels<N>::x_r2c, &CtKernels<N>::x_c2r},
+   &CtKernels<N>::x_eos, &CtKernels<N>::x_r2c, &CtKernels<N>::x_c2r, &CtKernels<N>::threads_per_line},
 const CtEntry kCtTable[] = {KWB_CT_SIZES(KWB_ENTRY)};
 #undef KWB_ENTRY
 
@@ -130,7 +131,8 @@ const CtEntry kRuntime = {0,
                           &CtKernels<0>::x_rho,
                           &CtKernels<0>::x_eos,
                           &CtKernels<0>::x_r2c,
-                          &CtKernels<0>::x_c2r};
+                          &CtKernels<0>::x_c2r,
+                          &CtKernels<0>::threads_per_line};
 
 // the kernels of transform length n: compile-time if listed, else runtime
 const CtEntry& kernels_for(int n) {
@@ -143,8 +145,17 @@ const CtEntry& kernels_for(int n) {
 
 bool ct_supported(int n) { return kernels_for(n).n == n && n > 0; }
 
-int col_lines(int n, int tl_rt) { return ct_supported(n) ? ct_lines_of(n) : tl_rt; }
-int row_lines_host(int n, int l_rt) { return ct_supported(n) ? ct_lines_of(n) : l_rt; }
+// The radix-plan variant (fft_ct.cuh) of `lines` transforms of length n per
+// pass: 1 where variant 0 would leave most of the device idle (fewer than 160
+// threads per SM).  us per step, variants 1 / 0 of every axis: 128 x 128
+// lossless (0.5 k threads a row pass) 25 / 51, 64 x 72 x 80 absorbing (12 k)
+// 96 / 129; of the x axis alone 1024 x 768 (25 k) 100 / 88, 128^3 (66 k)
+// 177 / 152.
+constexpr long long kNarrowThreads = 148 * 160;
+int plan_variant(int n, long long lines) {
+  if (!ct_supported(n)) return 0;
+  return lines * kernels_for(n).threads_per_line() < kNarrowThreads ? 1 : 0;
+}
 
 cudaError_t launch_col_fft(bool inv, const ColArgs& a, int nfields, long long nouter, const FFTPlan& plan,
                            const float2* tw, cudaStream_t st) {

@@ -20,6 +20,7 @@ struct Dims {
   long long nrows;  // ny * nz
   long long npts;   // nx * ny * nz
   long long row0, row1;  // rows [row0, row1) processed by a row-kernel launch
+  int v;            // radix-plan variant of the x transforms (fft_ct.cuh)
 };
 
 enum SpecOpKind {
@@ -134,6 +135,7 @@ struct ColArgs {
   long long lstride;  // element stride along the transformed axis
   long long ostride;  // stride of the outer index (blockIdx.y)
   int tl;             // columns per tile
+  int v;              // radix-plan variant
 };
 
 struct FusedArgs {
@@ -146,6 +148,7 @@ struct FusedArgs {
   int ncols;
   long long lstride, ostride;
   int tl;
+  int v;  // radix-plan variant
 };
 
 struct UArgs {

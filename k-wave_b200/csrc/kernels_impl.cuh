@@ -19,6 +19,8 @@
 // folded to constants); NC == 0 is the runtime-plan engine for any other
 // 2^a 3^b 5^c length.
 #pragma once
+#include <type_traits>
+
 #include "fft_ct.cuh"
 #include "kernels.cuh"
 #include "spec_ops.cuh"
@@ -26,51 +28,84 @@
 
 namespace kwb {
 
-// Lines per block / threads per block of a kernel instantiation.
-template <int NC>
+// Lines per block / threads per block of a column-kernel instantiation.
+template <int NC, int V>
 struct Tile {
-  static constexpr int LINES = ct_lines_of(NC);
-  static constexpr int THREADS = NC > 0 ? ct_threads_of(NC) : kThreads;
+  static constexpr int LINES = ct_col_lines(NC, Ct<NC, V>::T);
+  static constexpr int THREADS = NC > 0 ? Ct<NC, V>::T * LINES : kThreads;
 };
-// Row (x) tiles use half as many lines: smaller blocks, more of them per SM,
-// so their load / transform / store phases overlap.
 // The row kernels' 4-wide epilogue loops and their spectrum load / store
 // loops run without unrolling: at 256 points per row this cut registers
 // (k_x_rho 118 -> 90, k_x_u 72 -> 64) and instruction-fetch stalls, and the
 // 256^3 step went from 1.43 to 1.36 ms against unroll factors of 2-4.
 constexpr int kRowLoopUnroll = 1;
 
-template <int NC>
+// Row (x) tiles: small blocks (about 128 threads), several per SM, so their
+// load / transform / store phases overlap.  V: the plan variant (Ct).
+template <int NC, int V>
 struct RTile {
-  static constexpr int LINES = NC > 0 ? (ct_lines_of(NC) / 2 > 0 ? ct_lines_of(NC) / 2 : 1) : 0;
-  static constexpr int THREADS = NC > 0 ? (NC / ct_rmax(NC)) * LINES : kThreads;
-  // blocks per SM the register budget is sized for (about 512 threads)
-  static constexpr int MIN_BLOCKS = THREADS <= 128 ? 4 : (THREADS <= 256 ? 2 : 1);
+  static constexpr int LINES = NC > 0 ? ct_row_lines(Ct<NC, V>::T, V) : 0;
+  static constexpr int THREADS = NC > 0 ? Ct<NC, V>::T * LINES : kThreads;
+  // blocks per SM the register budgets of k_x_rho (about 512 threads, 384
+  // where a stage holds more than 16 elements a thread) and k_x_eos (about
+  // 640 and 512) are sized for
+  static constexpr bool HEAVY = Ct<NC, V>::held() > 16;
+  static constexpr int blocks(int threads) { return threads / THREADS > 0 ? threads / THREADS : 1; }
+  static constexpr int MIN_BLOCKS = blocks(HEAVY ? 384 : 512);
+  static constexpr int EOS_BLOCKS = NC > 0 ? blocks(HEAVY ? 512 : 640) : 0;  // 0: no bound
 };
 
-// Transform the lines of a tile.  Compile-time lengths run in place in `a`;
-// the runtime engine ping-pongs with `b`.  Returns the result buffer.
-template <int NC, bool INV, bool COL, class L>
-__device__ __forceinline__ float2* tile_fft(float2* a, float2* b, const float2* __restrict__ tw,
-                                            const FFTPlan& plan, int nlines, L lay) {
+// The row tile layout of an instantiation: CtRow for a compile-time length.
+template <int NC, int V>
+__device__ __forceinline__ auto row_lay(int nx) {
+  if constexpr (NC > 0)
+    return CtRow<NC, V>{};
+  else
+    return RowLayout{row_layout_stride(nx)};
+}
+template <int NC, int V>
+__host__ __device__ __forceinline__ int row_stride(int nx) {
+  if constexpr (NC > 0)
+    return CtRow<NC, V>::LS;
+  else
+    return row_layout_stride(nx);
+}
+
+// Transform the lines of a row tile.  Compile-time lengths run in place in
+// `a`; the runtime engine ping-pongs with `b`.  Returns the result buffer.
+template <int NC, int V, bool INV, class L>
+__device__ __forceinline__ float2* row_fft(float2* a, float2* b, const float2* __restrict__ tw, const FFTPlan& plan,
+                                           int nlines, L lay) {
   if constexpr (NC > 0) {
-    ct_fft<NC, INV, COL, Tile<NC>::LINES>(a, tw, lay);
+    ct_fft<NC, V, INV, false, RTile<NC, V>::LINES>(a, tw, lay);
     return a;
   } else {
-    return fft_lines<INV, COL>(a, b, tw, plan, nlines, lay);
+    return fft_lines<INV, false>(a, b, tw, plan, nlines, lay);
+  }
+}
+
+// The same for a column tile.
+template <int NC, int V, bool INV>
+__device__ __forceinline__ float2* col_fft(float2* a, float2* b, const float2* __restrict__ tw, const FFTPlan& plan,
+                                           int nlines) {
+  if constexpr (NC > 0) {
+    ct_fft<NC, V, INV, true, Tile<NC, V>::LINES>(a, tw, CtCol<Tile<NC, V>::LINES>{});
+    return a;
+  } else {
+    return fft_lines<INV, true>(a, b, tw, plan, nlines, ColLayout{nlines});
   }
 }
 
 // ---------------------------------------------------------------------------
 // column passes
 // ---------------------------------------------------------------------------
-template <int NC, bool INV>
-__global__ void __launch_bounds__(Tile<NC>::THREADS) k_col_fft(ColArgs a, const __grid_constant__ FFTPlan plan,
+template <int NC, int V, bool INV>
+__global__ void __launch_bounds__(Tile<NC, V>::THREADS) k_col_fft(ColArgs a, const __grid_constant__ FFTPlan plan,
                                                                const float2* __restrict__ tw_g) {
   extern __shared__ __align__(16) float2 sm[];
   constexpr bool CT = NC > 0;
   const int n = CT ? NC : plan.n;
-  const int tl = CT ? Tile<NC>::LINES : a.tl;
+  const int tl = CT ? Tile<NC, V>::LINES : a.tl;
   float2* tw = sm;
   float2* b0 = sm + n;
   float2* b1 = CT ? nullptr : b0 + tl * n;
@@ -84,7 +119,7 @@ __global__ void __launch_bounds__(Tile<NC>::THREADS) k_col_fft(ColArgs a, const 
     b0[i] = (c < a.ncols) ? g[p * a.lstride + c] : make_float2(0.f, 0.f);
   }
   __syncthreads();
-  float2* r = tile_fft<NC, INV, true>(b0, b1, tw, plan, tl, ColLayout{tl});
+  float2* r = col_fft<NC, V, INV>(b0, b1, tw, plan, tl);
 #pragma unroll 4
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int l = i % tl, p = i / tl, c = c0 + l;
@@ -94,15 +129,15 @@ __global__ void __launch_bounds__(Tile<NC>::THREADS) k_col_fft(ColArgs a, const 
 
 // Last axis: forward transform, multiply by `fanout` operators, inverse
 // transform each product.
-template <int NC>
-__global__ void __launch_bounds__(Tile<NC>::THREADS) k_fused_last(const __grid_constant__ FusedArgs a,
+template <int NC, int V>
+__global__ void __launch_bounds__(Tile<NC, V>::THREADS) k_fused_last(const __grid_constant__ FusedArgs a,
                                                                   const __grid_constant__ FFTPlan plan,
                                                                   const float2* __restrict__ tw_g,
                                                                   const __grid_constant__ SpecTables T, int dim) {
   extern __shared__ __align__(16) float2 sm[];
   constexpr bool CT = NC > 0;
   const int n = CT ? NC : plan.n;
-  const int tl = CT ? Tile<NC>::LINES : a.tl;
+  const int tl = CT ? Tile<NC, V>::LINES : a.tl;
   float2* tw = sm;
   float2* A = sm + n;
   float2* B = A + tl * n;
@@ -120,8 +155,7 @@ __global__ void __launch_bounds__(Tile<NC>::THREADS) k_fused_last(const __grid_c
     A[i] = (c < a.ncols) ? src[p * a.lstride + c] : make_float2(0.f, 0.f);
   }
   __syncthreads();
-  const ColLayout lay{tl};
-  float2* F = tile_fft<NC, false, true>(A, B, tw, plan, tl, lay);
+  float2* F = col_fft<NC, V, false>(A, B, tw, plan, tl);
   float2* W1 = (F == A) ? B : A;
   float2* W2 = C;
   for (int o = 0; o < a.fanout; ++o) {
@@ -135,7 +169,7 @@ __global__ void __launch_bounds__(Tile<NC>::THREADS) k_fused_last(const __grid_c
       W1[i] = c_mul(F[i], eval_op(op, T, dim, c, iy, iz));
     }
     __syncthreads();
-    float2* R = tile_fft<NC, true, true>(W1, W2, tw, plan, tl, lay);
+    float2* R = col_fft<NC, V, true>(W1, W2, tw, plan, tl);
     float2* dst = a.out[g * a.fanout + o] + off;
     float2* dst2 = a.dual_out[g * a.fanout + o];
     const float2 dsc = dst2 ? __ldg(a.dual_tab[g * a.fanout + o] + outer) : make_float2(0.f, 0.f);
@@ -156,11 +190,13 @@ __global__ void __launch_bounds__(Tile<NC>::THREADS) k_fused_last(const __grid_c
 // row (x axis) helpers.  A row tile holds 2L consecutive rows packed two per
 // complex line (row 2l in the real part, row 2l+1 in the imaginary part).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float get_comp(const float2* b, RowLayout lay, int q, int x) {
+template <class L>
+__device__ __forceinline__ float get_comp(const float2* b, L lay, int q, int x) {
   const float2& v = b[lay(q >> 1, x)];
   return (q & 1) ? v.y : v.x;
 }
-__device__ __forceinline__ void set_comp(float2* b, RowLayout lay, int q, int x, float v) {
+template <class L>
+__device__ __forceinline__ void set_comp(float2* b, L lay, int q, int x, float v) {
   float* f = reinterpret_cast<float*>(b + lay(q >> 1, x));
   f[q & 1] = v;
 }
@@ -168,8 +204,8 @@ __device__ __forceinline__ void set_comp(float2* b, RowLayout lay, int q, int x,
 // Build the full complex spectrum of each packed line from two half spectra
 // (C2R).  The imaginary parts of the k = 0 and Nyquist bins are dropped,
 // which is the Hermitian projection that real(ifftn(.)) performs.
-template <int NC>
-__device__ __forceinline__ void load_c2r(const float2* __restrict__ S, float2* buf, RowLayout lay, const Dims& d,
+template <int NC, class LAY>
+__device__ __forceinline__ void load_c2r(const float2* __restrict__ S, float2* buf, LAY lay, const Dims& d,
                                          long long r0, int L, const float2* __restrict__ kmul = nullptr,
                                          const float2* __restrict__ S2 = nullptr) {
   if constexpr (NC > 0 && NC % 4 == 0) {
@@ -247,8 +283,8 @@ __device__ __forceinline__ void load_c2r(const float2* __restrict__ S, float2* b
 
 // Split each packed line's spectrum Z = FFT(a + i b) into the half spectra
 // of a and b (R2C) and store them.
-template <int NC>
-__device__ __forceinline__ void store_r2c(const float2* buf, float2* __restrict__ S, RowLayout lay, const Dims& d,
+template <int NC, class LAY>
+__device__ __forceinline__ void store_r2c(const float2* buf, float2* __restrict__ S, LAY lay, const Dims& d,
                                           long long r0, int L) {
   if constexpr (NC > 0 && NC % 4 == 0) {
     constexpr int n = NC, nh = NC / 2 + 1, np = NC / 4 + 1;
@@ -446,7 +482,8 @@ __device__ __forceinline__ void sensor_dense4(const Sensor& s, int fi, long long
 }
 
 // Sparse sensors (mode 2) of a row tile, values read from the packed buffer.
-static __device__ void sensor_sparse_tile(const Sensor& s, int fi, const float2* buf, RowLayout lay, const Dims& d,
+template <class LAY>
+static __device__ void sensor_sparse_tile(const Sensor& s, int fi, const float2* buf, LAY lay, const Dims& d,
                                    long long r0, int L, int* sh) {
   if (s.mode != 2 || fi <= 0) return;
   const long long rend = min(r0 + 2LL * L, d.row1);
@@ -466,9 +503,29 @@ __device__ __forceinline__ float src_value(const SparseSource& s, const float* s
   return s.weight ? __ldg(s.weight + j) * v : v;
 }
 
-template <int NC>
+// Unit u of a row tile's 4-wide epilogue: 4 consecutive points (q, x .. x + 3).
+// Neighbouring threads take the same points of the two rows packed in a line
+// (its real and imaginary parts), so a warp's shared-memory accesses meet at
+// most one other in a bank.
+// (Where the layout is padded every 16 points they already do with whole rows
+// one after the other, which measured faster at 256 points: 1.19 against 1.20
+// ms per 256^3 step.)
+template <int NC, int V>
+__device__ __forceinline__ void row_unit(int u, int& q, int& x) {
+  constexpr int Q = NC / 4;
+  if constexpr (CtRow<NC, V>::SH == 4) {
+    q = u / Q;
+    x = 4 * (u - q * Q);
+  } else {
+    const int p = u >> 1, l = p / Q;
+    x = 4 * (p - l * Q);
+    q = 2 * l + (u & 1);
+  }
+}
+
+template <int NC, int V>
 __device__ __forceinline__ int row_lines(int L) {
-  return NC > 0 ? RTile<NC>::LINES : L;
+  return NC > 0 ? RTile<NC, V>::LINES : L;
 }
 
 // ---------------------------------------------------------------------------
@@ -530,11 +587,14 @@ struct TilePrefetch {
 // multiples), 2 nxp <= the packed line stride (the raw rows fit the buffer),
 // and buffers at 16-byte boundaries (an even lines x stride product).
 // ---------------------------------------------------------------------------
-template <int NC>
+template <int NC, int V>
 struct RowBulk {
-  static constexpr int LS = NC + NC / 16 + 1;  // row_layout_stride(NC)
-  static constexpr bool OK = NC > 0 && NC % 4 == 0 && 2 * (NC / 2 + 2) <= LS &&
-                             (RTile<NC>::LINES * LS) % 2 == 0 && NC % 2 == 0;
+  static constexpr int LS = CtRow<NC, V>::LS;
+  static constexpr bool OK = NC % 4 == 0 && 2 * (NC / 2 + 2) <= LS && (RTile<NC, V>::LINES * LS) % 2 == 0;
+};
+template <int V>
+struct RowBulk<0, V> {
+  static constexpr bool OK = false;
 };
 
 __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
@@ -614,8 +674,8 @@ struct RawRows {
 // general one to 72 (7 blocks); other lengths keep the compiler's own
 // choice (a minimum block count of 0 sets no bound), which caps would push
 // into spills (96, 128, 160, 192 points).
-template <int NC, bool LEAN>
-__global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7) : 0)
+template <int NC, int V, bool LEAN>
+__global__ void __launch_bounds__(RTile<NC, V>::THREADS, NC == 256 ? (LEAN ? 8 : 7) : 0)
     k_x_u(const __grid_constant__ UArgs a, Dims d,
                                                            const __grid_constant__ FFTPlan plan,
                                                            const float2* __restrict__ tw_g, int Lrt) {
@@ -623,16 +683,16 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
   __shared__ int sh[2];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC>(Lrt);
+  const int L = row_lines<NC, V>(Lrt);
   const int ax = blockIdx.y;
-  const RowLayout lay{row_layout_stride(nx)};
+  const auto lay = row_lay<NC, V>(nx);
   float2* tw = sm;
   float2* B0 = sm + nx;
-  float2* B1 = CT ? nullptr : B0 + L * lay.ls;
+  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, V>(nx);
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   __shared__ uint64_t rbar[1];
-  if constexpr (RowBulk<NC>::OK) {
+  if constexpr (RowBulk<NC, V>::OK) {
     if (threadIdx.x == 0) {
       mbar_init(&rbar[0], 1);
       fence_mbar_init();
@@ -640,7 +700,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
   }
   pdl_wait();  // everything below reads or writes the predecessors' data
   pdl_trigger();
-  if constexpr (RowBulk<NC>::OK) {  // the tile's spectrum rows are requested first
+  if constexpr (RowBulk<NC, V>::OK) {  // the tile's spectrum rows are requested first
     __syncthreads();
     if (threadIdx.x < 32) bulk_rows(B0, a.S[ax], d, r0, tile_rows(d, r0, L), &rbar[0]);
   }
@@ -648,7 +708,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
   const int fi = LEAN ? 0 : record_index(a.clk);
   const bool init = !LEAN && a.init;
   float2* G;
-  if constexpr (RowBulk<NC>::OK) {
+  if constexpr (RowBulk<NC, V>::OK) {
     {  // the epilogue's inputs stream in during the wait and the FFT
       TilePrefetch pf(d, r0, L);
       if (!init) pf.field(a.u[ax]);
@@ -659,7 +719,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
       drain_rows(rbar, 0, 1, a.wait);
       return;
     }
-    ct_fft_rows_ld<NC, true>(B0, tw, lay, RawRows<NC>{B0, d.nxp, tile_rows(d, r0, L), a.kmul[ax]});
+    ct_fft_rows_ld<NC, V, true>(B0, tw, lay, RawRows<NC>{B0, d.nxp, tile_rows(d, r0, L), a.kmul[ax]});
     G = B0;
   } else {
     load_c2r<NC>(a.S[ax], B0, lay, d, r0, L, a.kmul[ax]);
@@ -670,7 +730,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
       pf.field(a.rinv[ax].p);
       pf.sensor(a.sens[ax], fi);
     }
-    G = tile_fft<NC, true, false>(B0, B1, tw, plan, L, lay);
+    G = row_fft<NC, V, true>(B0, B1, tw, plan, L, lay);
   }
   float2* W = (G == B0) ? B1 : B0;
   float* u = a.u[ax];
@@ -684,8 +744,9 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
   if constexpr (VEC) {
     // 4 consecutive points per iteration, 16-byte global accesses
 #pragma unroll (kRowLoopUnroll)
-    for (int i = 4 * threadIdx.x; i < total; i += 4 * blockDim.x) {
-      const int q = i / nx, x = i - q * nx;
+    for (int i = threadIdx.x; i < total / 4; i += blockDim.x) {
+      int q, x;
+      row_unit<NC, V>(i, q, x);
       const long long row = r0 + q;
       if (row >= d.row1) {
 #pragma unroll
@@ -762,8 +823,9 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
   const Sensor& s = a.sens[ax];
   if constexpr (VEC) {
 #pragma unroll (kRowLoopUnroll)
-    for (int i = 4 * threadIdx.x; i < total; i += 4 * blockDim.x) {
-      const int q = i / nx, x = i - q * nx;
+    for (int i = threadIdx.x; i < total / 4; i += blockDim.x) {
+      int q, x;
+      row_unit<NC, V>(i, q, x);
       const long long row = r0 + q;
       if (row >= d.row1) continue;
       const long long gi = row * nx + x;
@@ -787,7 +849,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
   if (!LEAN) sensor_sparse_tile(s, fi, G, lay, d, r0, L, sh);
   if (a.do_r2c) {
     __syncthreads();
-    float2* F = tile_fft<NC, false, false>(G, W, tw, plan, L, lay);
+    float2* F = row_fft<NC, V, false>(G, W, tw, plan, L, lay);
     store_r2c<NC>(F, a.Sout[ax], lay, d, r0, L);
   }
 }
@@ -801,28 +863,28 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, NC == 256 ? (LEAN ? 8 : 7)
 // EOSK 1: the variant for power-law absorption without sparse pressure
 // sources (no sensor, Stokes, lossless-EOS or source-pass code: a smaller
 // kernel body); -1: every case, the equation of state read from a.eos.
-template <int NC, int DIM, int EOSK>
-__global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x_rho(const __grid_constant__ RhoArgs a, Dims d,
+template <int NC, int V, int DIM, int EOSK>
+__global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::MIN_BLOCKS) k_x_rho(const __grid_constant__ RhoArgs a, Dims d,
                                                              const __grid_constant__ FFTPlan plan,
                                                              const float2* __restrict__ tw_g, int Lrt) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ int sh[2];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC>(Lrt);
+  const int L = row_lines<NC, V>(Lrt);
   constexpr int dim = DIM;
   const int eos = EOSK >= 0 ? EOSK : a.eos;
-  const RowLayout lay{row_layout_stride(nx)};
+  const auto lay = row_lay<NC, V>(nx);
   float2* tw = sm;
   float2* pool[4];
-  for (int b = 0; b < 4; ++b) pool[b] = sm + nx + b * L * lay.ls;
+  for (int b = 0; b < 4; ++b) pool[b] = sm + nx + b * L * row_stride<NC, V>(nx);
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   // every divergence component's spectrum rows are requested first (not on
   // axisymmetric grids, whose u_r / r spectrum is summed in as S[1] is read)
   __shared__ uint64_t rbar[3];
-  const bool bulk = RowBulk<NC>::OK && !a.S_rr;
-  if constexpr (RowBulk<NC>::OK) {
+  const bool bulk = RowBulk<NC, V>::OK && !a.S_rr;
+  if constexpr (RowBulk<NC, V>::OK) {
     if (bulk && threadIdx.x == 0) {
       _Pragma("unroll") for (int f = 0; f < dim; ++f) mbar_init(&rbar[f], 1);
       fence_mbar_init();
@@ -830,7 +892,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x
   }
   pdl_wait();  // everything below reads or writes the predecessors' data
   pdl_trigger();
-  if constexpr (RowBulk<NC>::OK) {
+  if constexpr (RowBulk<NC, V>::OK) {
     if (bulk) {
       __syncthreads();
       if (threadIdx.x < 32) {
@@ -870,17 +932,17 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x
           if (eos != 1) pf.sensor(a.sens, fi);
         }
       }
-      if constexpr (RowBulk<NC>::OK) {
+      if constexpr (RowBulk<NC, V>::OK) {
         if (bulk) {
           if (!rows_ready(&rbar[f], a.wait)) {
             drain_rows(rbar, f, dim, a.wait);
             return;
           }
-          ct_fft_rows_ld<NC, true>(pool[f], tw, lay, RawRows<NC>{pool[f], d.nxp, tile_rows(d, r0, L), nullptr});
+          ct_fft_rows_ld<NC, V, true>(pool[f], tw, lay, RawRows<NC>{pool[f], d.nxp, tile_rows(d, r0, L), nullptr});
           continue;
         }
       }
-      tile_fft<NC, true, false>(pool[f], nullptr, tw, plan, L, lay);
+      row_fft<NC, V, true>(pool[f], nullptr, tw, plan, L, lay);
     }
     _Pragma("unroll") for (int f = 0; f < dim; ++f) D[f] = pool[f];
   } else {
@@ -897,7 +959,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x
       }
       load_c2r<NC>(a.S[f], pool[ia], lay, d, r0, L, nullptr, f == 1 ? a.S_rr : nullptr);
       __syncthreads();
-      D[f] = tile_fft<NC, true, false>(pool[ia], pool[ib], tw, plan, L, lay);
+      D[f] = row_fft<NC, V, true>(pool[ia], pool[ib], tw, plan, L, lay);
       used[(D[f] == pool[ia]) ? ia : ib] = true;
     }
     _Pragma("unroll") for (int b = 0; b <= dim; ++b)
@@ -914,8 +976,9 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x
   if (VEC && !sp) {
     // 4 consecutive points per iteration, 16-byte global accesses
 #pragma unroll (kRowLoopUnroll)
-    for (int i = 4 * threadIdx.x; i < total; i += 4 * blockDim.x) {
-      const int q = i / nx, x = i - q * nx;
+    for (int i = threadIdx.x; i < total / 4; i += blockDim.x) {
+      int q, x;
+      row_unit<NC, V>(i, q, x);
       const long long row = r0 + q;
       if (row >= d.row1) {
 #pragma unroll
@@ -1112,21 +1175,21 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x
 #pragma unroll 1
       for (int f = 0; f < 2; ++f) {
         if (f) __syncthreads();
-        tile_fft<NC, false, false>(D[f], nullptr, tw, plan, L, lay);
+        row_fft<NC, V, false>(D[f], nullptr, tw, plan, L, lay);
         store_r2c<NC>(D[f], f == 0 ? a.S_q : a.S_r, lay, d, r0, L);
       }
     } else {
-      float2* F = tile_fft<NC, false, false>(D[0], Wk, tw, plan, L, lay);
+      float2* F = row_fft<NC, V, false>(D[0], Wk, tw, plan, L, lay);
       store_r2c<NC>(F, a.S_q, lay, d, r0, L);
       __syncthreads();
       float2* Wk2 = (F == D[0]) ? Wk : D[0];
-      F = tile_fft<NC, false, false>(D[1], Wk2, tw, plan, L, lay);
+      F = row_fft<NC, V, false>(D[1], Wk2, tw, plan, L, lay);
       store_r2c<NC>(F, a.S_r, lay, d, r0, L);
     }
   } else {
     sensor_sparse_tile(a.sens, fi, D[0], lay, d, r0, L, sh);
     __syncthreads();
-    float2* F = tile_fft<NC, false, false>(D[0], Wk, tw, plan, L, lay);
+    float2* F = row_fft<NC, V, false>(D[0], Wk, tw, plan, L, lay);
     store_r2c<NC>(F, a.S_p, lay, d, r0, L);
   }
 }
@@ -1134,24 +1197,24 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS, RTile<NC>::MIN_BLOCKS) k_x
 // ---------------------------------------------------------------------------
 // power-law absorbing EOS: p = p_loc + c0^2 tau A - c0^2 eta B, sensors, R2C.
 // ---------------------------------------------------------------------------
-template <int NC>
-__global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_constant__ EosArgs a, Dims d,
+template <int NC, int V>
+__global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::EOS_BLOCKS) k_x_eos(const __grid_constant__ EosArgs a, Dims d,
                                                              const __grid_constant__ FFTPlan plan,
                                                              const float2* __restrict__ tw_g, int Lrt) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ int sh[2];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC>(Lrt);
-  const RowLayout lay{row_layout_stride(nx)};
+  const int L = row_lines<NC, V>(Lrt);
+  const auto lay = row_lay<NC, V>(nx);
   float2* tw = sm;
   float2* P0 = sm + nx;
-  float2* P1 = P0 + L * lay.ls;
-  float2* P2 = CT ? nullptr : P1 + L * lay.ls;
+  float2* P1 = P0 + L * row_stride<NC, V>(nx);
+  float2* P2 = CT ? nullptr : P1 + L * row_stride<NC, V>(nx);
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   __shared__ uint64_t rbar[2];
-  if constexpr (RowBulk<NC>::OK) {
+  if constexpr (RowBulk<NC, V>::OK) {
     if (threadIdx.x == 0) {
       mbar_init(&rbar[0], 1);
       mbar_init(&rbar[1], 1);
@@ -1160,7 +1223,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
   }
   pdl_wait();  // everything below reads or writes the predecessors' data
   pdl_trigger();
-  if constexpr (RowBulk<NC>::OK) {  // both spectra's rows are requested first
+  if constexpr (RowBulk<NC, V>::OK) {  // both spectra's rows are requested first
     __syncthreads();
     if (threadIdx.x < 32) {
       const int rows = tile_rows(d, r0, L);
@@ -1170,7 +1233,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
   }
   const int fi = record_index(a.clk);
   float2 *RA, *RB, *Wk;
-  if constexpr (RowBulk<NC>::OK) {
+  if constexpr (RowBulk<NC, V>::OK) {
     {  // the epilogue's inputs stream in during the waits and the FFTs
       TilePrefetch pf(d, r0, L);
       pf.field(a.p_loc);
@@ -1185,7 +1248,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
         return;
       }
       float2* P = f ? P1 : P0;
-      ct_fft_rows_ld<NC, true>(P, tw, lay, RawRows<NC>{P, d.nxp, tile_rows(d, r0, L), nullptr});
+      ct_fft_rows_ld<NC, V, true>(P, tw, lay, RawRows<NC>{P, d.nxp, tile_rows(d, r0, L), nullptr});
     }
     RA = P0;
     RB = P1;
@@ -1202,18 +1265,18 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
       pf.sensor(a.sens, fi);
     }
 #pragma unroll 1
-    for (int f = 0; f < 2; ++f) tile_fft<NC, true, false>(f ? P1 : P0, nullptr, tw, plan, L, lay);
+    for (int f = 0; f < 2; ++f) row_fft<NC, V, true>(f ? P1 : P0, nullptr, tw, plan, L, lay);
     RA = P0;
     RB = P1;
     Wk = nullptr;
   } else {
     load_c2r<NC>(a.S_a, P0, lay, d, r0, L);
     __syncthreads();
-    RA = tile_fft<NC, true, false>(P0, P1, tw, plan, L, lay);
+    RA = row_fft<NC, V, true>(P0, P1, tw, plan, L, lay);
     float2* f1 = (RA == P0) ? P1 : P0;
     load_c2r<NC>(a.S_b, f1, lay, d, r0, L);
     __syncthreads();
-    RB = tile_fft<NC, true, false>(f1, P2, tw, plan, L, lay);
+    RB = row_fft<NC, V, true>(f1, P2, tw, plan, L, lay);
     Wk = (RB == f1) ? P2 : f1;
   }
   const int total = 2 * L * nx;
@@ -1228,8 +1291,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
       bool ok;
     };
     auto load = [&](int i, In& v) {
-      v.q = i / nx;
-      v.x = i - v.q * nx;
+      row_unit<NC, V>(i, v.q, v.x);
       const long long row = r0 + v.q;
       v.ok = row < d.row1;
       if (!v.ok) return;
@@ -1260,7 +1322,7 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
     // (issuing two iterations' loads together measured the same: 1.2622
     // against 1.2616 ms per 256^3 step, at 113 instead of 72 registers)
 #pragma unroll 1
-    for (int i = 4 * threadIdx.x; i < total; i += 4 * blockDim.x) {
+    for (int i = threadIdx.x; i < total / 4; i += blockDim.x) {
       In v;
       load(i, v);
       update(v);
@@ -1286,25 +1348,25 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_eos(const __grid_const
   __syncthreads();
   sensor_sparse_tile(a.sens, fi, RA, lay, d, r0, L, sh);
   __syncthreads();
-  float2* F = tile_fft<NC, false, false>(RA, Wk, tw, plan, L, lay);
+  float2* F = row_fft<NC, V, false>(RA, Wk, tw, plan, L, lay);
   store_r2c<NC>(F, a.S_p, lay, d, r0, L);
 }
 
 // ---------------------------------------------------------------------------
 // plain x transforms (setup work, sources with k-space correction)
 // ---------------------------------------------------------------------------
-template <int NC>
-__global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_r2c(const float* __restrict__ f, float2* S, Dims d,
+template <int NC, int V>
+__global__ void __launch_bounds__(RTile<NC, V>::THREADS) k_x_r2c(const float* __restrict__ f, float2* S, Dims d,
                                                              const __grid_constant__ FFTPlan plan,
                                                              const float2* __restrict__ tw_g, int Lrt) {
   extern __shared__ __align__(16) float2 sm[];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC>(Lrt);
-  const RowLayout lay{row_layout_stride(nx)};
+  const int L = row_lines<NC, V>(Lrt);
+  const auto lay = row_lay<NC, V>(nx);
   float2* tw = sm;
   float2* B0 = sm + nx;
-  float2* B1 = CT ? nullptr : B0 + L * lay.ls;
+  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, V>(nx);
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   const int total = 2 * L * nx;
@@ -1314,29 +1376,29 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_r2c(const float* __res
     set_comp(B0, lay, q, x, row < d.row1 ? f[row * nx + x] : 0.f);
   }
   __syncthreads();
-  float2* F = tile_fft<NC, false, false>(B0, B1, tw, plan, L, lay);
+  float2* F = row_fft<NC, V, false>(B0, B1, tw, plan, L, lay);
   store_r2c<NC>(F, S, lay, d, r0, L);
 }
 
 // out = v (accumulate == 0) or out += v
-template <int NC>
-__global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_c2r(const float2* __restrict__ S, float* out,
+template <int NC, int V>
+__global__ void __launch_bounds__(RTile<NC, V>::THREADS) k_x_c2r(const float2* __restrict__ S, float* out,
                                                              int accumulate, Dims d,
                                                              const __grid_constant__ FFTPlan plan,
                                                              const float2* __restrict__ tw_g, int Lrt) {
   extern __shared__ __align__(16) float2 sm[];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC>(Lrt);
-  const RowLayout lay{row_layout_stride(nx)};
+  const int L = row_lines<NC, V>(Lrt);
+  const auto lay = row_lay<NC, V>(nx);
   float2* tw = sm;
   float2* B0 = sm + nx;
-  float2* B1 = CT ? nullptr : B0 + L * lay.ls;
+  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, V>(nx);
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   load_c2r<NC>(S, B0, lay, d, r0, L);
   __syncthreads();
-  float2* G = tile_fft<NC, true, false>(B0, B1, tw, plan, L, lay);
+  float2* G = row_fft<NC, V, true>(B0, B1, tw, plan, L, lay);
   const int total = 2 * L * nx;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int q = i / nx, x = i - q * nx;
@@ -1356,8 +1418,9 @@ __global__ void __launch_bounds__(RTile<NC>::THREADS) k_x_c2r(const float2* __re
 // (generated at build time), so the lengths compile in parallel.
 // ---------------------------------------------------------------------------
 static inline size_t smem_col(int n, int tl, int nbuf) { return sizeof(float2) * ((size_t)n + (size_t)nbuf * tl * n); }
+template <int NC, int V>
 static inline size_t smem_row(int nx, int L, int nbuf) {
-  return sizeof(float2) * ((size_t)nx + (size_t)nbuf * L * row_layout_stride(nx));
+  return sizeof(float2) * ((size_t)nx + (size_t)nbuf * L * row_stride<NC, V>(nx));
 }
 
 template <class K>
@@ -1367,84 +1430,84 @@ static inline void set_smem(K k, size_t sm) {
 
 static inline unsigned row_tiles(const Dims& d, int L) { return (unsigned)((d.row1 - d.row0 + 2 * L - 1) / (2 * L)); }
 
-template <int NC, bool INV>
+template <int NC, int V, bool INV>
 static void col_fft_t(const ColArgs& a0, int nfields, long long nouter, const FFTPlan& plan, const float2* tw,
                       cudaStream_t st) {
   ColArgs a = a0;
-  const int tl = NC > 0 ? Tile<NC>::LINES : a.tl;
+  const int tl = NC > 0 ? Tile<NC, V>::LINES : a.tl;
   a.tl = tl;
   dim3 grid((a.ncols + tl - 1) / tl, (unsigned)nouter, nfields);
   const size_t sm = smem_col(plan.n, tl, NC > 0 ? 1 : 2);
-  set_smem(k_col_fft<NC, INV>, sm);
-  k_col_fft<NC, INV><<<grid, Tile<NC>::THREADS, sm, st>>>(a, plan, tw);
+  set_smem(k_col_fft<NC, V, INV>, sm);
+  k_col_fft<NC, V, INV><<<grid, Tile<NC, V>::THREADS, sm, st>>>(a, plan, tw);
 }
 
-template <int NC>
+template <int NC, int V>
 static void fused_t(const FusedArgs& a0, int ninputs, long long nouter, const FFTPlan& plan, const float2* tw,
                     const SpecTables& T, int dim, cudaStream_t st) {
   FusedArgs a = a0;
-  const int tl = NC > 0 ? Tile<NC>::LINES : a.tl;
+  const int tl = NC > 0 ? Tile<NC, V>::LINES : a.tl;
   a.tl = tl;
   dim3 grid((a.ncols + tl - 1) / tl, (unsigned)nouter, ninputs);
   const size_t sm = smem_col(plan.n, tl, NC > 0 ? 2 : 3);
-  set_smem(k_fused_last<NC>, sm);
-  k_fused_last<NC><<<grid, Tile<NC>::THREADS, sm, st>>>(a, plan, tw, T, dim);
+  set_smem(k_fused_last<NC, V>, sm);
+  k_fused_last<NC, V><<<grid, Tile<NC, V>::THREADS, sm, st>>>(a, plan, tw, T, dim);
 }
 
-template <int NC>
+template <int NC, int V>
 static void x_u_t(const UArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int Lrt, cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC>::LINES : Lrt;
-  const size_t sm = smem_row(d.nx, L, NC > 0 ? 1 : 2);
+  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
+  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 1 : 2);
   bool lean = !a.init && a.src.n == 0;
   for (int ax = 0; ax < d.dim; ++ax) lean = lean && !a.dsrc[ax].field && a.sens[ax].mode == 0;
   auto go = [&](auto k) {
     set_smem(k, sm);
-    launch_pdl(k, dim3(row_tiles(d, L), d.dim), dim3(RTile<NC>::THREADS), sm, st, a, d, plan, tw, L);
+    launch_pdl(k, dim3(row_tiles(d, L), d.dim), dim3(RTile<NC, V>::THREADS), sm, st, a, d, plan, tw, L);
   };
-  lean ? go(k_x_u<NC, true>) : go(k_x_u<NC, false>);
+  lean ? go(k_x_u<NC, V, true>) : go(k_x_u<NC, V, false>);
 }
 
-template <int NC>
+template <int NC, int V>
 static void x_rho_t(const RhoArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int Lrt,
                     cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC>::LINES : Lrt;
-  const size_t sm = smem_row(d.nx, L, NC > 0 ? d.dim : d.dim + 1);
+  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
+  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? d.dim : d.dim + 1);
   auto go = [&](auto k) {
     set_smem(k, sm);
-    launch_pdl(k, dim3(row_tiles(d, L)), dim3(RTile<NC>::THREADS), sm, st, a, d, plan, tw, L);
+    launch_pdl(k, dim3(row_tiles(d, L)), dim3(RTile<NC, V>::THREADS), sm, st, a, d, plan, tw, L);
   };
   const bool lean = a.eos == 1 && a.src.n == 0;
   if (d.dim == 3)
-    lean ? go(k_x_rho<NC, 3, 1>) : go(k_x_rho<NC, 3, -1>);
+    lean ? go(k_x_rho<NC, V, 3, 1>) : go(k_x_rho<NC, V, 3, -1>);
   else
-    lean ? go(k_x_rho<NC, 2, 1>) : go(k_x_rho<NC, 2, -1>);
+    lean ? go(k_x_rho<NC, V, 2, 1>) : go(k_x_rho<NC, V, 2, -1>);
 }
 
-template <int NC>
+template <int NC, int V>
 static void x_eos_t(const EosArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int Lrt,
                     cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC>::LINES : Lrt;
-  const size_t sm = smem_row(d.nx, L, NC > 0 ? 2 : 3);
-  set_smem(k_x_eos<NC>, sm);
-  launch_pdl(k_x_eos<NC>, dim3(row_tiles(d, L)), dim3(RTile<NC>::THREADS), sm, st, a, d, plan, tw, L);
+  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
+  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 2 : 3);
+  set_smem(k_x_eos<NC, V>, sm);
+  launch_pdl(k_x_eos<NC, V>, dim3(row_tiles(d, L)), dim3(RTile<NC, V>::THREADS), sm, st, a, d, plan, tw, L);
 }
 
-template <int NC>
+template <int NC, int V>
 static void x_r2c_t(const float* f, float2* S, const Dims& d, const FFTPlan& plan, const float2* tw, int Lrt,
                     cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC>::LINES : Lrt;
-  const size_t sm = smem_row(d.nx, L, NC > 0 ? 1 : 2);
-  set_smem(k_x_r2c<NC>, sm);
-  k_x_r2c<NC><<<row_tiles(d, L), RTile<NC>::THREADS, sm, st>>>(f, S, d, plan, tw, L);
+  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
+  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 1 : 2);
+  set_smem(k_x_r2c<NC, V>, sm);
+  k_x_r2c<NC, V><<<row_tiles(d, L), RTile<NC, V>::THREADS, sm, st>>>(f, S, d, plan, tw, L);
 }
 
-template <int NC>
+template <int NC, int V>
 static void x_c2r_t(const float2* S, float* out, int acc, const Dims& d, const FFTPlan& plan, const float2* tw,
                     int Lrt, cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC>::LINES : Lrt;
-  const size_t sm = smem_row(d.nx, L, NC > 0 ? 1 : 2);
-  set_smem(k_x_c2r<NC>, sm);
-  k_x_c2r<NC><<<row_tiles(d, L), RTile<NC>::THREADS, sm, st>>>(S, out, acc, d, plan, tw, L);
+  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
+  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 1 : 2);
+  set_smem(k_x_c2r<NC, V>, sm);
+  k_x_c2r<NC, V><<<row_tiles(d, L), RTile<NC, V>::THREADS, sm, st>>>(S, out, acc, d, plan, tw, L);
 }
 
 // The launchers of one length.  Member functions are defined out of class
@@ -1465,45 +1528,58 @@ struct CtKernels {
                     cudaStream_t st);
   static void x_c2r(const float2* S, float* out, int acc, const Dims& d, const FFTPlan& plan, const float2* tw,
                     int L, cudaStream_t st);
+  static int threads_per_line() { return Ct<NC, 0>::T; }  // variant 0
 };
+
+// f(integral_constant<V>) for the plan variant v (the runtime-plan engine
+// has only variant 0).
+template <int NC, class F>
+static inline void with_variant(int v, F&& f) {
+  if constexpr (NC > 0) {
+    if (v) return f(std::integral_constant<int, 1>{});
+  }
+  f(std::integral_constant<int, 0>{});
+}
 
 template <int NC>
 void CtKernels<NC>::col_fft(bool inv, const ColArgs& a, int nfields, long long nouter, const FFTPlan& plan,
                             const float2* tw, cudaStream_t st) {
-  if (inv)
-    col_fft_t<NC, true>(a, nfields, nouter, plan, tw, st);
-  else
-    col_fft_t<NC, false>(a, nfields, nouter, plan, tw, st);
+  with_variant<NC>(a.v, [&](auto v) {
+    if (inv)
+      col_fft_t<NC, v.value, true>(a, nfields, nouter, plan, tw, st);
+    else
+      col_fft_t<NC, v.value, false>(a, nfields, nouter, plan, tw, st);
+  });
 }
 template <int NC>
 void CtKernels<NC>::fused(const FusedArgs& a, int ninputs, long long nouter, const FFTPlan& plan,
                           const float2* tw, const SpecTables& T, int dim, cudaStream_t st) {
-  fused_t<NC>(a, ninputs, nouter, plan, tw, T, dim, st);
+  with_variant<NC>(a.v, [&](auto v) { fused_t<NC, v.value>(a, ninputs, nouter, plan, tw, T, dim, st); });
 }
 template <int NC>
 void CtKernels<NC>::x_u(const UArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                         cudaStream_t st) {
-  x_u_t<NC>(a, d, plan, tw, L, st);
+  with_variant<NC>(d.v, [&](auto v) { x_u_t<NC, v.value>(a, d, plan, tw, L, st); });
 }
 template <int NC>
 void CtKernels<NC>::x_rho(const RhoArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                           cudaStream_t st) {
-  x_rho_t<NC>(a, d, plan, tw, L, st);
+  with_variant<NC>(d.v, [&](auto v) { x_rho_t<NC, v.value>(a, d, plan, tw, L, st); });
 }
 template <int NC>
 void CtKernels<NC>::x_eos(const EosArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                           cudaStream_t st) {
-  x_eos_t<NC>(a, d, plan, tw, L, st);
+  with_variant<NC>(d.v, [&](auto v) { x_eos_t<NC, v.value>(a, d, plan, tw, L, st); });
 }
 template <int NC>
 void CtKernels<NC>::x_r2c(const float* f, float2* S, const Dims& d, const FFTPlan& plan, const float2* tw,
                           int L, cudaStream_t st) {
-  x_r2c_t<NC>(f, S, d, plan, tw, L, st);
+  with_variant<NC>(d.v, [&](auto v) { x_r2c_t<NC, v.value>(f, S, d, plan, tw, L, st); });
 }
 template <int NC>
 void CtKernels<NC>::x_c2r(const float2* S, float* out, int acc, const Dims& d, const FFTPlan& plan,
                           const float2* tw, int L, cudaStream_t st) {
-  x_c2r_t<NC>(S, out, acc, d, plan, tw, L, st);
+  with_variant<NC>(d.v, [&](auto v) { x_c2r_t<NC, v.value>(S, out, acc, d, plan, tw, L, st); });
 }
 
 }  // namespace kwb

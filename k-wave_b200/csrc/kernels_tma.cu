@@ -30,11 +30,11 @@ namespace kwb {
 // 1.336 ms per step).
 constexpr int kColStages = 3;
 
-template <int NC, bool INV>
-__global__ void __launch_bounds__(TTile<NC>::THREADS) k_col_tma(const __grid_constant__ ColTmaArgs a,
+template <int NC, int V, bool INV>
+__global__ void __launch_bounds__(TTile<NC, V>::THREADS) k_col_tma(const __grid_constant__ ColTmaArgs a,
                                                                 const float2* __restrict__ tw_g) {
-  constexpr int TL = TTile<NC>::LINES;
-  constexpr int E = TTile<NC>::STRIDE;  // stage stride (the tile, padded to 128 bytes)
+  constexpr int TL = TTile<NC, V>::LINES;
+  constexpr int E = TTile<NC, V>::STRIDE;  // stage stride (the tile, padded to 128 bytes)
   constexpr int ST = kColStages;
   extern __shared__ __align__(128) unsigned char smraw[];
   float2* bufs = reinterpret_cast<float2*>(smraw);
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS) k_col_tma(const __grid_con
     const int s = j % ST;
     int f, x, y, z;
     coords(t, f, x, y, z);
-    mbar_expect_tx(&bar[s], TTile<NC>::BYTES);
+    mbar_expect_tx(&bar[s], TTile<NC, V>::BYTES);
     if (t == a.wait.skip_tile) return;  // test hook: announced, never issued
     tma_load_3d(bufs + s * E, &a.map[f == a.dual_field ? a.dual_src : f], x, y, z, &bar[s]);
     inflight |= 1u << s;
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS) k_col_tma(const __grid_con
     if (t0 >= 0) issue(t0, 0);
     if (t1 >= 0) issue(t1, 1);
   }
-  const ColLayout lay{TL};
+  const CtCol<TL> lay{};
   bool aborted = false;
   for (int it = 0;; ++it) {
     const int t = tile_at(it);
@@ -114,10 +114,10 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS) k_col_tma(const __grid_con
     if (f == a.dual_field) {  // the derived field: the first stage reads its input times the axis factor
       const int l = threadIdx.x % TL, tid = threadIdx.x / TL;
       const float2* tab = a.dual_tab;
-      ct_stage0_ld<NC, INV>(b, l, tid, lay, [&](int ll, int n) { return c_mul(b[lay(ll, n)], __ldg(tab + n)); });
-      ct_stages<NC, 1, INV>(b, tw, l, tid, lay);
+      ct_stage0_ld<NC, V, INV>(b, l, tid, lay, [&](int ll, int n) { return c_mul(b[lay(ll, n)], __ldg(tab + n)); });
+      ct_stages<NC, V, 1, Ct<NC, V>::S, INV, false>(b, tw, l, tid, lay);
     } else {
-      ct_fft<NC, INV, true, TL>(b, tw, lay);
+      ct_fft<NC, V, INV, true, TL>(b, tw, lay);
     }
     fence_async_smem();
     __syncthreads();
@@ -142,6 +142,18 @@ __global__ void __launch_bounds__(TTile<NC>::THREADS) k_col_tma(const __grid_con
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+int tma_lines(int n, int v) {
+  switch (n) {
+#define KWB_CASE(N) \
+  case N:           \
+    return v ? TTile<N, 1>::LINES : TTile<N, 0>::LINES;
+    KWB_TMA_COL_SIZES(KWB_CASE)
+#undef KWB_CASE
+    default:
+      return 0;
+  }
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
 static bool get_encoder() {
@@ -173,9 +185,9 @@ bool tma_fused_supported(int n) { return tma_col_supported(n); }
 // of a row is loaded with zeros past bin nxh - 1 and stored clipped there,
 // so padding costs no memory traffic.  Tiles start at x = cx * lines, a
 // multiple of 16 bytes.
-bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n) {
+bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n, int v) {
   if (!get_encoder()) return false;
-  const int lines = tma_lines_of(n);
+  const int lines = tma_lines(n, v);
   if (d.nxp % 2 != 0 || (lines * 8) % 16 != 0 || lines > 256 || n > 256) return false;
   cuuint64_t dims[3] = {(cuuint64_t)d.nxh, (cuuint64_t)d.ny, (cuuint64_t)d.nz};
   cuuint64_t strides[2] = {(cuuint64_t)d.nxp * 8, (cuuint64_t)d.nxp * d.ny * 8};
@@ -213,26 +225,25 @@ int tma_num_sms() {
   return g_num_sms;
 }
 
-template <int NC, bool INV>
+template <int NC, int V, bool INV>
 static cudaError_t col_tma_t(const ColTmaArgs& a, const float2* tw, cudaStream_t st) {
-  const size_t sm = kColStages * TTile<NC>::STRIDE * sizeof(float2) + NC * sizeof(float2) + kColStages * sizeof(uint64_t);
-  auto k = k_col_tma<NC, INV>;
+  const size_t sm = kColStages * TTile<NC, V>::STRIDE * sizeof(float2) + NC * sizeof(float2) + kColStages * sizeof(uint64_t);
+  auto k = k_col_tma<NC, V, INV>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TTile<NC>::THREADS, sm);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TTile<NC, V>::THREADS, sm);
   const int ntiles = a.nfields * a.ncx * a.nouter;
   const int grid = std::min(ntiles, std::max(1, per_sm) * tma_num_sms());
-  const cudaError_t e = launch_pdl(k, dim3(grid), dim3(TTile<NC>::THREADS), sm, st, a, tw);
+  const cudaError_t e = launch_pdl(k, dim3(grid), dim3(TTile<NC, V>::THREADS), sm, st, a, tw);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
-
-int tma_lines(int n) { return tma_lines_of(n); }
 
 cudaError_t launch_col_tma(bool inv, int n, const ColTmaArgs& a, const float2* tw, cudaStream_t st) {
   switch (n) {
 #define KWB_CASE(N) \
   case N:           \
-    return inv ? col_tma_t<N, true>(a, tw, st) : col_tma_t<N, false>(a, tw, st);
+    return a.v ? (inv ? col_tma_t<N, 1, true>(a, tw, st) : col_tma_t<N, 1, false>(a, tw, st)) \
+               : (inv ? col_tma_t<N, 0, true>(a, tw, st) : col_tma_t<N, 0, false>(a, tw, st));
     KWB_TMA_COL_SIZES(KWB_CASE)
 #undef KWB_CASE
     default:

@@ -18,6 +18,7 @@ struct TmaWaitArgs {
 struct ColTmaArgs {
   CUtensorMap map[4];  // one per field; box {LINES, N, 1} (y pass) or {LINES, 1, N} (last axis)
   int nfields;
+  int v;        // radix-plan variant (tile shape and transform)
   int ncx;      // column tiles along kx
   int nouter;   // outer extent of this launch (z planes for the y pass)
   int outer0;   // first outer index
@@ -43,6 +44,7 @@ struct FusedTmaArgs {
   long long lstride;    // element stride along the transformed axis
   long long ostride;    // stride of the outer index
   int nin, fanout, ncx, nouter, yaxis, dim;
+  int v;      // radix-plan variant (tile shape and transform)
   int ncols;  // valid kx columns (nx / 2 + 1)
   // Remainder tiles (3D): when the last column kx = ncols - 1 would be alone
   // in its column tile, it is gathered for rem_y consecutive outer indices

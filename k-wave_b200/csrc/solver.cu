@@ -65,8 +65,9 @@ cudaError_t launch_medium_maps(float* c0_to_c0sq, float c0_scalar, float* ctau, 
 cudaError_t launch_reciprocal(float* v, long long n, cudaStream_t st);
 bool tma_col_supported(int n);    // TMA-fed y pass
 bool tma_fused_supported(int n);  // TMA-fed fused last-axis operator
-int tma_lines(int n);
-bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n);
+int tma_lines(int n, int v);
+int plan_variant(int n, long long lines);
+bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n, int v);
 bool make_spec_map_rem(CUtensorMap* m, void* base, const Dims& d, int n, int rows);
 cudaError_t launch_col_tma(bool inv, int n, const ColTmaArgs& a, const float2* tw, cudaStream_t st);
 cudaError_t launch_fused_tma(int n, const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st);
@@ -465,6 +466,12 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
   }
   rowL = std::max(1, std::min(8, 2048 / d.nx));
 
+  // radix-plan variant per axis: from the lines of a whole-volume pass, so it
+  // does not depend on the launch schedule
+  plan_v[0] = d.v = plan_variant(d.nx, (d.nrows + 1) / 2);
+  plan_v[1] = plan_variant(d.ny, (long long)d.nxh * d.nz);
+  plan_v[2] = d.dim == 3 ? plan_variant(d.nz, (long long)d.nxh * d.ny) : 0;
+
   // ----- operator tables -----
   const double dd[3] = {in->dx, in->dy, in->dz};
   const double dt = in->dt, c_ref = in->c_ref;
@@ -651,13 +658,13 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
   use_tma[1] = tma_ok && (d.dim == 3 ? tma_col_supported(d.ny) : tma_fused_supported(d.ny));
   use_tma[2] = tma_ok && d.dim == 3 && tma_fused_supported(d.nz);
   for (int s = 0; s < nspec; ++s) {
-    if (use_tma[1] && !make_spec_map(&map_y[s], S_buf[s].p, d, 1, d.ny)) use_tma[1] = false;
-    if (use_tma[2] && !make_spec_map(&map_z[s], S_buf[s].p, d, 2, d.nz)) use_tma[2] = false;
+    if (use_tma[1] && !make_spec_map(&map_y[s], S_buf[s].p, d, 1, d.ny, plan_v[1])) use_tma[1] = false;
+    if (use_tma[2] && !make_spec_map(&map_z[s], S_buf[s].p, d, 2, d.nz, plan_v[2])) use_tma[2] = false;
   }
   // last-axis remainder tiles: when kx = nx / 2 would be alone in its column
   // tile, it is gathered for TL / 2 consecutive y into one tile instead
   {
-    const int tl = use_tma[2] ? tma_lines(d.nz) : 0;
+    const int tl = use_tma[2] ? tma_lines(d.nz, plan_v[2]) : 0;
     rem_y = tl / 2;
     use_rem = use_tma[2] && tl % 2 == 0 && (d.nxh - 1) % tl == 0 && (d.nxh - 1) % 2 == 0 && d.ny % rem_y == 0;
     for (int s = 0; s < nspec && use_rem; ++s)
@@ -889,7 +896,8 @@ void Session::col_pass(bool inv, const std::vector<int>& bufs, int z0, int nzs, 
     ca.dual_src = dual_src;
     ca.dual_tab = dual_tab;
     ca.nfields = n;
-    ca.ncx = (d.nxh + tma_lines(d.ny) - 1) / tma_lines(d.ny);
+    ca.v = plan_v[1];
+    ca.ncx = (d.nxh + tma_lines(d.ny, plan_v[1]) - 1) / tma_lines(d.ny, plan_v[1]);
     ca.nouter = nzs;
     ca.outer0 = z0;
     ca.yaxis = 1;
@@ -904,6 +912,7 @@ void Session::col_pass(bool inv, const std::vector<int>& bufs, int z0, int nzs, 
     ca.lstride = d.nxp;
     ca.ostride = (long long)d.nxp * d.ny;
     ca.tl = col_tl[1];
+    ca.v = plan_v[1];
     ck(launch_col_fft(inv, ca, n, nzs, plan[1], twd[1], st), "col_fft");
   }
   ++launches_;
@@ -935,11 +944,12 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
     fa.lstride = (long long)d.nxp * (d.dim == 3 ? d.ny : 1);
     fa.ostride = d.nxp;
     fa.nin = nin;
+    fa.v = plan_v[last];
     fa.fanout = fanout;
-    fa.ncx = (d.nxh + tma_lines(ns[last]) - 1) / tma_lines(ns[last]);
+    fa.ncx = (d.nxh + tma_lines(ns[last], plan_v[last]) - 1) / tma_lines(ns[last], plan_v[last]);
     fa.nouter = (d.dim == 3) ? d.ny : 1;
     if (d.dim == 3 && use_rem) {
-      fa.ncx = (d.nxh - 1) / tma_lines(ns[last]);
+      fa.ncx = (d.nxh - 1) / tma_lines(ns[last], plan_v[last]);
       fa.nrem = d.ny / rem_y;
       fa.rem_y = rem_y;
       for (int i = 0; i < nin; ++i) fa.in_rem[i] = map_zr[ins[i]];
@@ -966,6 +976,7 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
     fa.lstride = (long long)d.nxp * (d.dim == 3 ? d.ny : 1);
     fa.ostride = d.nxp;
     fa.tl = col_tl[last];
+    fa.v = plan_v[last];
     ck(launch_fused_last(fa, nin, d.dim == 3 ? d.ny : 1, plan[last], twd[last], T, d.dim, st), "fused_last");
   }
   ++launches_;

@@ -127,6 +127,7 @@ class Session {
   int col_tl[3]{16, 16, 16};
   int col_tl_max[3]{16, 16, 16};
   int rowL = 8;
+  int plan_v[3]{0, 0, 0};  // radix-plan variant of each axis (fft_ct.cuh)
   int slab = 1;  // z planes per chain slab
   Schedule sched_{};
   const kw_input* in_user = nullptr;  // the caller's input (before any axisymmetric expansion)
