@@ -51,33 +51,33 @@ def _run(cmd):
     return r
 
 
-def ct_sizes():
-    """Transform lengths listed in csrc/ct_sizes.h."""
+def _lengths(header):
+    """Transform lengths listed in a csrc/*_sizes.h header."""
     import re
 
-    with open(os.path.join(CSRC, "ct_sizes.h")) as f:
+    with open(os.path.join(CSRC, header)) as f:
         return [int(v) for v in re.findall(r"X\((\d+)\)", f.read())]
+
+
+def ct_sizes():
+    """Transform lengths listed in csrc/ct_sizes.h."""
+    return _lengths("ct_sizes.h")
 
 
 def tma_sizes():
     """Transform lengths listed in csrc/tma_sizes.h."""
-    import re
-
-    with open(os.path.join(CSRC, "tma_sizes.h")) as f:
-        return [int(v) for v in re.findall(r"X\((\d+)\)", f.read())]
+    return _lengths("tma_sizes.h")
 
 
-def _fused_sources():
-    """One generated translation unit per TMA length: an explicit
-    instantiation of the fused last-axis pass fused_tma_cls<N> (fused_tma.cuh)."""
-    d = os.path.join(BUILD, "tma")
+def _generated(sub, prefix, header, kernels, lengths):
+    """One generated translation unit per length, an explicit instantiation of
+    `kernels`<N>; heaviest (longest) lengths first."""
+    d = os.path.join(BUILD, sub)
     os.makedirs(d, exist_ok=True)
     out = []
-    for n in tma_sizes():
-        path = os.path.join(d, f"fused_tma_{n}.cu")
-        text = (f'#include "fused_tma.cuh"\nnamespace kwb {{\n'
-                f'template cudaError_t fused_tma_cls<{n}>(const FusedTmaArgs&, const float2*, const SpecTables&,'
-                f' cudaStream_t);\n}}\n')
+    for n in sorted(lengths, reverse=True):
+        path = os.path.join(d, f"{prefix}_{n}.cu")
+        text = f'#include "{header}"\nnamespace kwb {{\ntemplate struct {kernels}<{n}>;\n}}\n'
         if not os.path.exists(path) or open(path).read() != text:
             with open(path, "w") as f:
                 f.write(text)
@@ -86,19 +86,15 @@ def _fused_sources():
 
 
 def _ct_sources():
-    """One generated translation unit per compile-time length: an explicit
-    instantiation of CtKernels<N> (kernels_impl.cuh)."""
-    d = os.path.join(BUILD, "ct")
-    os.makedirs(d, exist_ok=True)
-    out = []
-    for n in ct_sizes():
-        path = os.path.join(d, f"kernels_ct_{n}.cu")
-        text = f'#include "kernels_impl.cuh"\nnamespace kwb {{\ntemplate struct CtKernels<{n}>;\n}}\n'
-        if not os.path.exists(path) or open(path).read() != text:
-            with open(path, "w") as f:
-                f.write(text)
-        out.append(path)
-    return out
+    """CtKernels<N> (kernels_impl.cuh): the row kernels and the plain y pass."""
+    return _generated("ct", "kernels_ct", "kernels_impl.cuh", "CtKernels",
+                      ct_sizes() + _lengths("ct_more_sizes.h"))
+
+
+def _tma_sources():
+    """TmaKernels<N> (fused_tma.cuh): the TMA-fed y pass and last-axis operator."""
+    return _generated("tma", "tma", "fused_tma.cuh", "TmaKernels",
+                      tma_sizes() + _lengths("tma_more_sizes.h") + _lengths("ct_more_sizes.h"))
 
 
 def build(force: bool = False, jobs: int = 0, verbose: bool = False) -> str:
@@ -107,7 +103,7 @@ def build(force: bool = False, jobs: int = 0, verbose: bool = False) -> str:
     hdrs = _headers()
     jobs_list = []
     objs = []
-    for s in _ct_sources() + _fused_sources():
+    for s in _ct_sources() + _tma_sources():
         o = s[:-3] + ".o"
         objs.append(o)
         if force or _stale(o, [s] + hdrs):

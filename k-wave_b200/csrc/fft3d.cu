@@ -38,7 +38,7 @@ cudaError_t launch_x_r2c(const float* f, float2* S, const Dims& d, const FFTPlan
                          cudaStream_t st);
 cudaError_t launch_x_c2r(const float2* S, float* out, int accumulate, const Dims& d, const FFTPlan& plan,
                          const float2* tw, int L, cudaStream_t st);
-bool tma_col_supported(int n);
+bool tma_supported(int n);
 int tma_lines(int n, int v);
 bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n, int v);
 cudaError_t launch_col_tma(bool inv, int n, const ColTmaArgs& a, const float2* tw, cudaStream_t st);
@@ -74,7 +74,7 @@ void fck(cudaError_t e, const char* what) {
 void column_pass(const kw_fft3d_plan& p, int axis, bool inv, float2* S, cudaStream_t st) {
   const Dims& d = p.d;
   const int n = axis == 1 ? d.ny : d.nz;
-  if (tma_col_supported(n)) {
+  if (tma_supported(n)) {
     ColTmaArgs ca;
     std::memset(&ca, 0, sizeof(ca));
     if (!make_spec_map(&ca.map[0], S, d, axis, n, ca.v)) throw std::runtime_error("tensor map of the spectrum");
@@ -83,7 +83,6 @@ void column_pass(const kw_fft3d_plan& p, int axis, bool inv, float2* S, cudaStre
     ca.ncx = (d.nxh + tma_lines(n, ca.v) - 1) / tma_lines(n, ca.v);
     ca.nouter = axis == 1 ? d.nz : d.ny;
     ca.outer0 = 0;
-    ca.yaxis = axis;
     ca.err = p.err;
     ca.wait = TmaWaitArgs{2000000000ull, -1};
     fck(launch_col_tma(inv, n, ca, p.tw[axis], st), "column pass");

@@ -116,6 +116,11 @@ struct Ct {
     }
     return h;
   }
+  static constexpr bool has7() {  // a radix-7 or radix-14 stage (the heaviest codelets)
+    for (int i = 0; i < P.s; ++i)
+      if (P.r[i] % 7 == 0) return true;
+    return false;
+  }
   static constexpr int radix(int stage, bool rev) { return rev ? P.r[S - 1 - stage] : P.r[stage]; }
   static constexpr int ns(int stage, bool rev) {  // product of the radices before `stage`
     int p = 1;

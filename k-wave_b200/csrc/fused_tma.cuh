@@ -1,46 +1,10 @@
 // The TMA-fed fused last-axis operator (forward transform, k-space operator
-// multiply, inverse transform) and the tile geometry it shares with the y
-// pass.  Templates only: each transform length is instantiated in its own
-// translation unit (fused_tma_N.cu, generated by build.py from tma_sizes.h).
+// multiply, inverse transform) and the launchers of one length.
 #pragma once
-#include <algorithm>
-
-#include "fft_ct.cuh"
-#include "kernels.cuh"
-#include "kernels_tma.cuh"
+#include "col_tma.cuh"
 #include "spec_ops.cuh"
-#include "tma.cuh"
-#include "tma_sizes.h"
 
 namespace kwb {
-
-int tma_num_sms();  // multiprocessors of the current device
-
-// Lines per TMA tile: the column tile's, a multiple of 4, so every tile starts
-// at a bin index x = cx * LINES whose byte offset (8-byte bins) is a multiple
-// of 32 (tensor copies require 16).
-template <int NC, int V>
-struct TTile {
-  static constexpr int LINES = ct_col_lines(NC, Ct<NC, V>::T);
-  static constexpr int THREADS = Ct<NC, V>::T * LINES;
-  static constexpr int ELEMS = LINES * NC;
-  static constexpr unsigned BYTES = ELEMS * sizeof(float2);
-  // Stage stride in elements: tensor copies read and write shared memory at
-  // 128-byte aligned addresses, so each stage is padded to a multiple of 128
-  // bytes.
-  static constexpr int STRIDE = (int)((BYTES + 127u) / 128u * 128u / sizeof(float2));
-};
-
-__device__ __forceinline__ void tile_coords(int yaxis, int cx, int o, int lines, int& x, int& y, int& z) {
-  x = cx * lines;
-  if (yaxis == 1) {
-    y = 0;
-    z = o;
-  } else {
-    y = o;
-    z = 0;
-  }
-}
 
 // Operator classes of the fused kernel: one instantiation per class keeps
 // only that operator's arithmetic in the kernel body.
@@ -48,11 +12,12 @@ enum FusedClass { FC_GRAD = 0, FC_NABLA = 1, FC_SRCK = 2 };
 
 // Blocks per SM the register budget is sized for: about 768 threads for the
 // single-output pass, 512 otherwise and where a stage holds more than 16
-// elements a thread (180 = 15 x 12 spilled 0.26 KB a thread at 768).
+// elements a thread or a radix is a multiple of 7 (180 = 15 x 12 spilled
+// 0.26 KB a thread at 768).
 template <int NC, int V, int MODE>
 struct FusedBounds {
   static constexpr int TH = TTile<NC, V>::THREADS;
-  static constexpr int WANT = MODE && Ct<NC, V>::held() <= 16 ? 768 : 512;
+  static constexpr int WANT = MODE && Ct<NC, V>::held() <= 16 && !Ct<NC, V>::has7() ? 768 : 512;
   static constexpr int MIN_BLOCKS = WANT / TH > 0 ? WANT / TH : 1;
 };
 
@@ -120,15 +85,14 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
   if (threadIdx.x == 0) inflight = parity_bits = 0;
   auto issue = [&](int t, int j) {  // tile t, consumed at loop iteration j
     const int s = j & 1;
-    int g, cx, o, x, y, z;
+    int g, cx, o;
     decode(t, g, cx, o);
     mbar_expect_tx(&bar[s], TTile<NC, V>::BYTES);  // a remainder box holds as many bytes
     if (t == a.wait.skip_tile) return;  // test hook: announced, never issued
     if (cx >= 0) {
-      tile_coords(a.yaxis, cx, o, TL, x, y, z);
-      tma_load_3d(inb + s * E, &a.in[g], x, y, z, &bar[s]);
+      tma_load_4d(inb + s * E, &a.in[g], cx * TL, 0, 0, o, &bar[s]);
     } else {
-      tma_load_3d(inb + s * E, &a.in_rem[g], a.ncols - 1, o, 0, &bar[s]);
+      tma_load_4d(inb + s * E, &a.in_rem[g], a.ncols - 1, o, 0, 0, &bar[s]);
     }
     inflight |= 1u << s;
     parity_bits = (parity_bits & ~(1u << s)) | ((unsigned)((j >> 1) & 1) << s);
@@ -140,8 +104,6 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
     if (blockIdx.x + gridDim.x < ntiles) issue(blockIdx.x + gridDim.x, 1);
   }
   const CtCol<TL> lay{};
-  // the line mapping fixes this thread's column (kx) for every pass
-  const int l = threadIdx.x % TL, tid = threadIdx.x / TL;
   const float cdt2sq = T.cdt2 * T.cdt2;
   constexpr int TPL = TH / TL;  // threads per line
   constexpr int M = CtHandoff<NC, V>::M;
@@ -151,6 +113,7 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
     const int s = it & 1;
     float2* F = inb + s * E;
+    const int id = ct_tid<NC>(tw), l = id % TL, tid = id / TL;
     int g, cx, o;
     decode(t, g, cx, o);
     // this thread's line: its column ix and outer index ol, where its
@@ -336,14 +299,29 @@ cudaError_t fused_tma_v(const FusedTmaArgs& a, const float2* tw, const SpecTable
   if (kind == OP_NABLA1 || kind == OP_NABLA2) return fused_tma_t<NC, V, FC_NABLA, 1>(a, tw, T, st);
   return fused_tma_t<NC, V, FC_SRCK, 1>(a, tw, T, st);
 }
+
+// The launchers of one length, on the plan variant the arguments name.
+// Member functions are defined out of class (so not inline): each length is
+// instantiated in its own translation unit (generated by build.py from
+// tma_sizes.h and tma_more_sizes.h).
 template <int NC>
-cudaError_t fused_tma_cls(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st) {
+struct TmaKernels {
+  static int lines(int v);  // columns per tile
+  static cudaError_t col(bool inv, const ColTmaArgs& a, const float2* tw, cudaStream_t st);
+  static cudaError_t fused(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st);
+};
+template <int NC>
+int TmaKernels<NC>::lines(int v) {
+  return v ? TTile<NC, 1>::LINES : TTile<NC, 0>::LINES;
+}
+template <int NC>
+cudaError_t TmaKernels<NC>::col(bool inv, const ColTmaArgs& a, const float2* tw, cudaStream_t st) {
+  if (a.v) return inv ? col_tma_t<NC, 1, true>(a, tw, st) : col_tma_t<NC, 1, false>(a, tw, st);
+  return inv ? col_tma_t<NC, 0, true>(a, tw, st) : col_tma_t<NC, 0, false>(a, tw, st);
+}
+template <int NC>
+cudaError_t TmaKernels<NC>::fused(const FusedTmaArgs& a, const float2* tw, const SpecTables& T, cudaStream_t st) {
   return a.v ? fused_tma_v<NC, 1>(a, tw, T, st) : fused_tma_v<NC, 0>(a, tw, T, st);
 }
-
-#define KWB_FUSED_EXTERN(N) \
-  extern template cudaError_t fused_tma_cls<N>(const FusedTmaArgs&, const float2*, const SpecTables&, cudaStream_t);
-KWB_TMA_COL_SIZES(KWB_FUSED_EXTERN)
-#undef KWB_FUSED_EXTERN
 
 }  // namespace kwb

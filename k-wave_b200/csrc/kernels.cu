@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "ct_more_sizes.h"
 #include "ct_sizes.h"
 #include "kernels_impl.cuh"
 
@@ -13,6 +14,7 @@ namespace kwb {
 
 #define KWB_EXTERN(N) extern template struct CtKernels<N>;
 KWB_CT_SIZES(KWB_EXTERN)
+KWB_CT_MORE_SIZES(KWB_EXTERN)
 #undef KWB_EXTERN
 
 // ---------------------------------------------------------------------------
@@ -101,6 +103,62 @@ __global__ void k_rms_final(const float2* __restrict__ acc, const float* __restr
     out[i] = sqrtf((acc[i].x + (partial ? blk[i] : 0.f)) * inv_n);
 }
 
+// Last axis without TMA: forward transform, multiply by `fanout` operators,
+// inverse transform each product (runtime-plan engine, any length).
+__global__ void __launch_bounds__(kThreads) k_fused_last(const __grid_constant__ FusedArgs a,
+                                                         const __grid_constant__ FFTPlan plan,
+                                                         const float2* __restrict__ tw_g,
+                                                         const __grid_constant__ SpecTables T, int dim) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int n = plan.n, tl = a.tl;
+  float2* tw = sm;
+  float2* A = sm + n;
+  float2* B = A + tl * n;
+  float2* C = B + tl * n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = tw_g[i];
+  const int g = blockIdx.z;
+  const int outer = blockIdx.y;
+  const long long off = (long long)outer * a.ostride;
+  const float2* src = a.in[g] + off;
+  const int c0 = blockIdx.x * tl;
+  const int total = tl * n;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int l = i % tl, p = i / tl, c = c0 + l;
+    A[i] = (c < a.ncols) ? src[p * a.lstride + c] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  const ColLayout lay{tl};
+  float2* F = fft_lines<false, true>(A, B, tw, plan, tl, lay);
+  float2* W1 = (F == A) ? B : A;
+  for (int o = 0; o < a.fanout; ++o) {
+    const SpecOp op = a.op[g * a.fanout + o];
+    for (int i = threadIdx.x; i < total; i += blockDim.x) {
+      const int l = i % tl, p = i / tl;
+      int c = c0 + l;
+      if (c >= a.ncols) c = 0;
+      const int iy = (dim == 3) ? outer : p;
+      const int iz = (dim == 3) ? p : 0;
+      W1[i] = c_mul(F[i], eval_op(op, T, dim, c, iy, iz));
+    }
+    __syncthreads();
+    float2* R = fft_lines<true, true>(W1, C, tw, plan, tl, lay);
+    float2* dst = a.out[g * a.fanout + o] + off;
+    float2* dst2 = a.dual_out[g * a.fanout + o];
+    const float2 dsc = dst2 ? __ldg(a.dual_tab[g * a.fanout + o] + outer) : make_float2(0.f, 0.f);
+    if (dst2) dst2 += off;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < total; i += blockDim.x) {
+      const int l = i % tl, p = i / tl, c = c0 + l;
+      if (c < a.ncols) {
+        dst[p * a.lstride + c] = R[i];
+        if (dst2) dst2[p * a.lstride + c] = c_mul(R[i], dsc);
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // ---------------------------------------------------------------------------
 // host-side launch helpers, dispatching on the transform length
 // ---------------------------------------------------------------------------
@@ -109,7 +167,6 @@ namespace {
 struct CtEntry {
   int n;
   decltype(&CtKernels<0>::col_fft) col_fft;
-  decltype(&CtKernels<0>::fused) fused;
   decltype(&CtKernels<0>::x_u) x_u;
   decltype(&CtKernels<0>::x_rho) x_rho;
   decltype(&CtKernels<0>::x_eos) x_eos;
@@ -119,14 +176,13 @@ struct CtEntry {
 };
 
 #define KWB_ENTRY(N)                                                                                  \
-  {N, &CtKernels<N>::col_fft, &CtKernels<N>::fused, &CtKernels<N>::x_u, &CtKernels<N>::x_rho,          \
+  {N, &CtKernels<N>::col_fft, &CtKernels<N>::x_u, &CtKernels<N>::x_rho,          \
    &CtKernels<N>::x_eos, &CtKernels<N>::x_r2c, &CtKernels<N>::x_c2r, &CtKernels<N>::threads_per_line},
-const CtEntry kCtTable[] = {KWB_CT_SIZES(KWB_ENTRY)};
+const CtEntry kCtTable[] = {KWB_CT_SIZES(KWB_ENTRY) KWB_CT_MORE_SIZES(KWB_ENTRY)};
 #undef KWB_ENTRY
 
 const CtEntry kRuntime = {0,
                           &CtKernels<0>::col_fft,
-                          &CtKernels<0>::fused,
                           &CtKernels<0>::x_u,
                           &CtKernels<0>::x_rho,
                           &CtKernels<0>::x_eos,
@@ -165,7 +221,10 @@ cudaError_t launch_col_fft(bool inv, const ColArgs& a, int nfields, long long no
 
 cudaError_t launch_fused_last(const FusedArgs& a, int ninputs, long long nouter, const FFTPlan& plan,
                               const float2* tw, const SpecTables& T, int dim, cudaStream_t st) {
-  kernels_for(plan.n).fused(a, ninputs, nouter, plan, tw, T, dim, st);
+  const dim3 grid((a.ncols + a.tl - 1) / a.tl, (unsigned)nouter, ninputs);
+  const size_t sm = smem_col(plan.n, a.tl, 3);
+  set_smem(k_fused_last, sm);
+  k_fused_last<<<grid, kThreads, sm, st>>>(a, plan, tw, T, dim);
   return cudaGetLastError();
 }
 

@@ -148,7 +148,6 @@ struct FusedArgs {
   int ncols;
   long long lstride, ostride;
   int tl;
-  int v;  // radix-plan variant
 };
 
 struct UArgs {

@@ -127,65 +127,6 @@ __global__ void __launch_bounds__(Tile<NC, V>::THREADS) k_col_fft(ColArgs a, con
   }
 }
 
-// Last axis: forward transform, multiply by `fanout` operators, inverse
-// transform each product.
-template <int NC, int V>
-__global__ void __launch_bounds__(Tile<NC, V>::THREADS) k_fused_last(const __grid_constant__ FusedArgs a,
-                                                                  const __grid_constant__ FFTPlan plan,
-                                                                  const float2* __restrict__ tw_g,
-                                                                  const __grid_constant__ SpecTables T, int dim) {
-  extern __shared__ __align__(16) float2 sm[];
-  constexpr bool CT = NC > 0;
-  const int n = CT ? NC : plan.n;
-  const int tl = CT ? Tile<NC, V>::LINES : a.tl;
-  float2* tw = sm;
-  float2* A = sm + n;
-  float2* B = A + tl * n;
-  float2* C = CT ? nullptr : B + tl * n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = tw_g[i];
-  const int g = blockIdx.z;
-  const int outer = blockIdx.y;
-  const long long off = (long long)outer * a.ostride;
-  const float2* src = a.in[g] + off;
-  const int c0 = blockIdx.x * tl;
-  const int total = tl * n;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
-    const int l = i % tl, p = i / tl, c = c0 + l;
-    A[i] = (c < a.ncols) ? src[p * a.lstride + c] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  float2* F = col_fft<NC, V, false>(A, B, tw, plan, tl);
-  float2* W1 = (F == A) ? B : A;
-  float2* W2 = C;
-  for (int o = 0; o < a.fanout; ++o) {
-    const SpecOp op = a.op[g * a.fanout + o];
-    for (int i = threadIdx.x; i < total; i += blockDim.x) {
-      const int l = i % tl, p = i / tl;
-      int c = c0 + l;
-      if (c >= a.ncols) c = 0;
-      const int iy = (dim == 3) ? outer : p;
-      const int iz = (dim == 3) ? p : 0;
-      W1[i] = c_mul(F[i], eval_op(op, T, dim, c, iy, iz));
-    }
-    __syncthreads();
-    float2* R = col_fft<NC, V, true>(W1, W2, tw, plan, tl);
-    float2* dst = a.out[g * a.fanout + o] + off;
-    float2* dst2 = a.dual_out[g * a.fanout + o];
-    const float2 dsc = dst2 ? __ldg(a.dual_tab[g * a.fanout + o] + outer) : make_float2(0.f, 0.f);
-    if (dst2) dst2 += off;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < total; i += blockDim.x) {
-      const int l = i % tl, p = i / tl, c = c0 + l;
-      if (c < a.ncols) {
-        dst[p * a.lstride + c] = R[i];
-        if (dst2) dst2[p * a.lstride + c] = c_mul(R[i], dsc);
-      }
-    }
-    __syncthreads();
-  }
-}
-
 // ---------------------------------------------------------------------------
 // row (x axis) helpers.  A row tile holds 2L consecutive rows packed two per
 // complex line (row 2l in the real part, row 2l+1 in the imaginary part).
@@ -1443,18 +1384,6 @@ static void col_fft_t(const ColArgs& a0, int nfields, long long nouter, const FF
 }
 
 template <int NC, int V>
-static void fused_t(const FusedArgs& a0, int ninputs, long long nouter, const FFTPlan& plan, const float2* tw,
-                    const SpecTables& T, int dim, cudaStream_t st) {
-  FusedArgs a = a0;
-  const int tl = NC > 0 ? Tile<NC, V>::LINES : a.tl;
-  a.tl = tl;
-  dim3 grid((a.ncols + tl - 1) / tl, (unsigned)nouter, ninputs);
-  const size_t sm = smem_col(plan.n, tl, NC > 0 ? 2 : 3);
-  set_smem(k_fused_last<NC, V>, sm);
-  k_fused_last<NC, V><<<grid, Tile<NC, V>::THREADS, sm, st>>>(a, plan, tw, T, dim);
-}
-
-template <int NC, int V>
 static void x_u_t(const UArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int Lrt, cudaStream_t st) {
   const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
   const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 1 : 2);
@@ -1517,8 +1446,6 @@ template <int NC>
 struct CtKernels {
   static void col_fft(bool inv, const ColArgs& a, int nfields, long long nouter, const FFTPlan& plan,
                       const float2* tw, cudaStream_t st);
-  static void fused(const FusedArgs& a, int ninputs, long long nouter, const FFTPlan& plan, const float2* tw,
-                    const SpecTables& T, int dim, cudaStream_t st);
   static void x_u(const UArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L, cudaStream_t st);
   static void x_rho(const RhoArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                     cudaStream_t st);
@@ -1550,11 +1477,6 @@ void CtKernels<NC>::col_fft(bool inv, const ColArgs& a, int nfields, long long n
     else
       col_fft_t<NC, v.value, false>(a, nfields, nouter, plan, tw, st);
   });
-}
-template <int NC>
-void CtKernels<NC>::fused(const FusedArgs& a, int ninputs, long long nouter, const FFTPlan& plan,
-                          const float2* tw, const SpecTables& T, int dim, cudaStream_t st) {
-  with_variant<NC>(a.v, [&](auto v) { fused_t<NC, v.value>(a, ninputs, nouter, plan, tw, T, dim, st); });
 }
 template <int NC>
 void CtKernels<NC>::x_u(const UArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,

@@ -16,13 +16,12 @@ struct TmaWaitArgs {
 };
 
 struct ColTmaArgs {
-  CUtensorMap map[4];  // one per field; box {LINES, N, 1} (y pass) or {LINES, 1, N} (last axis)
+  CUtensorMap map[4];  // one per field (make_spec_map)
   int nfields;
   int v;        // radix-plan variant (tile shape and transform)
   int ncx;      // column tiles along kx
   int nouter;   // outer extent of this launch (z planes for the y pass)
   int outer0;   // first outer index
-  int yaxis;    // 1: the transformed axis is the tensor's y dimension, 2: z
   // Optional derived field (dual_field >= 0): its tiles are loaded from
   // field dual_src, multiplied by dual_tab[position along the transformed
   // axis] and transformed, then stored to its own map.  Tiles are then dealt
@@ -43,12 +42,12 @@ struct FusedTmaArgs {
   const float2* dual_tab[9];
   long long lstride;    // element stride along the transformed axis
   long long ostride;    // stride of the outer index
-  int nin, fanout, ncx, nouter, yaxis, dim;
+  int nin, fanout, ncx, nouter, dim;
   int v;      // radix-plan variant (tile shape and transform)
   int ncols;  // valid kx columns (nx / 2 + 1)
   // Remainder tiles (3D): when the last column kx = ncols - 1 would be alone
   // in its column tile, it is gathered for rem_y consecutive outer indices
-  // into one tile instead (box {2, rem_y, n}, lines alternating kx = ncols - 1
+  // into one tile instead (make_spec_map_rem, lines alternating kx = ncols - 1
   // and the zero-filled padding bin), so the ncx column tiles stop at
   // ncols - 1.  nrem: remainder tiles per input (0: none).
   CUtensorMap in_rem[3];

@@ -63,8 +63,7 @@ cudaError_t launch_medium_maps(float* c0_to_c0sq, float c0_scalar, float* ctau, 
                                float alpha_scalar, double np_per_db, double y, double tan_py, int eos, long long n,
                                cudaStream_t st);
 cudaError_t launch_reciprocal(float* v, long long n, cudaStream_t st);
-bool tma_col_supported(int n);    // TMA-fed y pass
-bool tma_fused_supported(int n);  // TMA-fed fused last-axis operator
+bool tma_supported(int n);  // TMA-fed y pass and fused last-axis operator
 int tma_lines(int n, int v);
 int plan_variant(int n, long long lines);
 bool make_spec_map(CUtensorMap* m, void* base, const Dims& d, int yaxis, int n, int v);
@@ -655,8 +654,8 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
   }
   if (const char* k = std::getenv("KWAVE_B200_TEST_SKIP_TMA_TILE")) tma_wait.skip_tile = std::atoi(k);
   // use_tma[1]: the y pass in 3D, the fused last-axis operator in 2D
-  use_tma[1] = tma_ok && (d.dim == 3 ? tma_col_supported(d.ny) : tma_fused_supported(d.ny));
-  use_tma[2] = tma_ok && d.dim == 3 && tma_fused_supported(d.nz);
+  use_tma[1] = tma_ok && tma_supported(d.ny);
+  use_tma[2] = tma_ok && d.dim == 3 && tma_supported(d.nz);
   for (int s = 0; s < nspec; ++s) {
     if (use_tma[1] && !make_spec_map(&map_y[s], S_buf[s].p, d, 1, d.ny, plan_v[1])) use_tma[1] = false;
     if (use_tma[2] && !make_spec_map(&map_z[s], S_buf[s].p, d, 2, d.nz, plan_v[2])) use_tma[2] = false;
@@ -900,7 +899,6 @@ void Session::col_pass(bool inv, const std::vector<int>& bufs, int z0, int nzs, 
     ca.ncx = (d.nxh + tma_lines(d.ny, plan_v[1]) - 1) / tma_lines(d.ny, plan_v[1]);
     ca.nouter = nzs;
     ca.outer0 = z0;
-    ca.yaxis = 1;
     ca.err = (int*)err_buf.p;
     ca.wait = tma_wait;
     ck(launch_col_tma(inv, d.ny, ca, twd[1], st), "col_tma");
@@ -954,7 +952,6 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
       fa.rem_y = rem_y;
       for (int i = 0; i < nin; ++i) fa.in_rem[i] = map_zr[ins[i]];
     }
-    fa.yaxis = (d.dim == 3) ? 2 : 1;
     fa.dim = d.dim;
     fa.ncols = d.nxh;
     fa.err = (int*)err_buf.p;
@@ -976,7 +973,6 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
     fa.lstride = (long long)d.nxp * (d.dim == 3 ? d.ny : 1);
     fa.ostride = d.nxp;
     fa.tl = col_tl[last];
-    fa.v = plan_v[last];
     ck(launch_fused_last(fa, nin, d.dim == 3 ? d.ny : 1, plan[last], twd[last], T, d.dim, st), "fused_last");
   }
   ++launches_;
