@@ -36,6 +36,7 @@
 
 #include "fft_engine.cuh"
 #include "kwave_b200.h"
+#include "tma.cuh"
 
 namespace {
 
@@ -43,10 +44,22 @@ using namespace kwb;
 
 constexpr int MAX_EDGE = KW_NOALLOC_MAX_EDGE;
 constexpr int MAX_NXH = MAX_EDGE / 2 + 1;
-constexpr int TL = 8;           // kx columns per CTA in the y pass
+constexpr int MAX_TL = 8;       // most kx columns per CTA in the y pass
+constexpr int MIN_COL_BLOCKS = 120;
 constexpr int THREADS = 256;
 // y pass: twiddles + three column tiles; x passes need far less
-constexpr size_t MAX_SMEM = sizeof(float2) * ((size_t)MAX_EDGE + 3ull * MAX_EDGE * TL);
+constexpr size_t MAX_SMEM = sizeof(float2) * ((size_t)MAX_EDGE + 3ull * MAX_EDGE * MAX_TL);
+
+// Columns per CTA in the y pass: the most that still give MIN_COL_BLOCKS CTAs.
+// The spectra (at most 4 MiB each) stay in L2, so the narrow rows of a small
+// tile cost no DRAM traffic, and a call is a chain of latencies: at 384 x 320
+// eight columns meant 25 CTAs with three transforms of 2560 elements one after
+// the other, 34 us of the call's 51.
+int col_tile(int nxh) {
+  int tl = MAX_TL;
+  while (tl > 1 && (nxh + tl - 1) / tl < MIN_COL_BLOCKS) tl /= 2;
+  return tl;
+}
 
 // Two half spectra of the largest grid: [component][ky][kx], kx fastest.
 static __device__ __align__(256) float2 g_scratch[2 * MAX_EDGE * MAX_NXH];
@@ -57,6 +70,7 @@ struct GradArgs {
   float2* S[2];      // half spectra in the scratch
   FFTPlan px, py;
   int nx, ny, nxh, ngrad;
+  int tl;            // kx columns per CTA in phase 1
   float kx_step, ky_step;  // 2 pi / (N d)
   float half_cdt;          // c_ref dt / 2
   float inv_n;             // 1 / (nx ny)
@@ -86,9 +100,11 @@ __device__ __forceinline__ float2 shifted_derivative(int m, int n, float kstep) 
 __device__ __forceinline__ float sinc(float x) { return x == 0.f ? 1.f : sinf(x) / x; }
 
 // Phase 0: R2C along x of row pairs into S[0].
-// Phase 1: along y per group of TL kx columns: forward FFT, multiply by
+// Phase 1: along y per group of tl kx columns: forward FFT, multiply by
 //          kappa and the two shifted derivatives, inverse FFTs into S[0], S[1].
 // Phase 2: C2R along x of S[c] into g[c] (blockIdx.y = component c).
+// The phases are launched with programmatic stream serialization: each builds
+// its twiddles while the one before ends (pdl_wait, tma.cuh).
 __global__ void __launch_bounds__(THREADS) k_grad2d_noalloc(GradArgs a, int phase) {
   extern __shared__ float2 sm[];
   if (phase == 0) {
@@ -98,6 +114,8 @@ __global__ void __launch_bounds__(THREADS) k_grad2d_noalloc(GradArgs a, int phas
     float2* b0 = tw + n;
     float2* b1 = b0 + L.ls;
     twiddles(tw, n);
+    pdl_wait();
+    pdl_trigger();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       const float re = a.f[(size_t)r * n + i];
       const float im = r + 1 < a.ny ? a.f[(size_t)(r + 1) * n + i] : 0.f;
@@ -112,6 +130,7 @@ __global__ void __launch_bounds__(THREADS) k_grad2d_noalloc(GradArgs a, int phas
       if (r + 1 < a.ny) a.S[0][(size_t)(r + 1) * a.nxh + m] = make_float2(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
     }
   } else if (phase == 1) {
+    const int TL = a.tl;
     const int n = a.ny, m0 = blockIdx.x * TL;
     const ColLayout C{TL};
     float2* tw = sm;
@@ -119,6 +138,8 @@ __global__ void __launch_bounds__(THREADS) k_grad2d_noalloc(GradArgs a, int phas
     float2* b1 = b0 + n * TL;
     float2* b2 = b1 + n * TL;
     twiddles(tw, n);
+    pdl_wait();
+    pdl_trigger();
     for (int i = threadIdx.x; i < n * TL; i += blockDim.x) {
       const int l = i % TL, j = i / TL, m = m0 + l;
       b0[C(l, j)] = m < a.nxh ? a.S[0][(size_t)j * a.nxh + m] : make_float2(0.f, 0.f);
@@ -159,6 +180,8 @@ __global__ void __launch_bounds__(THREADS) k_grad2d_noalloc(GradArgs a, int phas
     float2* b0 = tw + n;
     float2* b1 = b0 + L.ls;
     twiddles(tw, n);
+    pdl_wait();
+    pdl_trigger();
     const bool pair = r + 1 < a.ny;
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       const bool direct = k < a.nxh;
@@ -223,7 +246,9 @@ extern "C" int kw_kspace_gradient_noalloc(const float* d_f, float* d_gx, float* 
                 "grid %llu x %llu is outside 2..%d per edge, the size of the static scratch",
                 (unsigned long long)nx, (unsigned long long)ny, MAX_EDGE);
   GradArgs a{};
-  if (!make_fft_plan((int)nx, &a.px) || !make_fft_plan((int)ny, &a.py))
+  // variant 2, no radix-16 stage: with one line or a few columns per CTA most
+  // threads would idle in one
+  if (!make_fft_plan((int)nx, &a.px, 2) || !make_fft_plan((int)ny, &a.py, 2))
     return fail(status, KW_ERR_UNSUPPORTED, "grid edges must be products of 2, 3, 5 and 7 (got %llu x %llu)",
                 (unsigned long long)nx, (unsigned long long)ny);
   if (!(dx > 0.f) || !(dy > 0.f) || !(dt > 0.f) || !(c_ref >= 0.f) || !std::isfinite(dx) || !std::isfinite(dy) ||
@@ -268,13 +293,16 @@ extern "C" int kw_kspace_gradient_noalloc(const float* d_f, float* d_gx, float* 
   a.half_cdt = 0.5f * c_ref * dt;
   a.inv_n = (float)(1.0 / ((double)NX * NY));
 
+  a.tl = col_tile(a.nxh);
   const size_t row_smem = sizeof(float2) * (NX + 2 * row_layout_stride(NX));
-  const size_t col_smem = sizeof(float2) * ((size_t)NY + 3ull * NY * TL);
+  const size_t col_smem = sizeof(float2) * ((size_t)NY + 3ull * NY * a.tl);
   const unsigned row_pairs = (unsigned)((NY + 1) / 2);
-  k_grad2d_noalloc<<<row_pairs, THREADS, row_smem, st>>>(a, 0);
-  k_grad2d_noalloc<<<(unsigned)((a.nxh + TL - 1) / TL), THREADS, col_smem, st>>>(a, 1);
-  k_grad2d_noalloc<<<dim3(row_pairs, (unsigned)a.ngrad), THREADS, row_smem, st>>>(a, 2);
-  e = cudaGetLastError();
+  e = launch_pdl(k_grad2d_noalloc, dim3(row_pairs), dim3(THREADS), row_smem, st, a, 0);
+  if (e == cudaSuccess)
+    e = launch_pdl(k_grad2d_noalloc, dim3((unsigned)((a.nxh + a.tl - 1) / a.tl)), dim3(THREADS), col_smem, st, a, 1);
+  if (e == cudaSuccess)
+    e = launch_pdl(k_grad2d_noalloc, dim3(row_pairs, (unsigned)a.ngrad), dim3(THREADS), row_smem, st, a, 2);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(status, KW_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
   return KW_OK;
 }
