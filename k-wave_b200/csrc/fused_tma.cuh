@@ -100,6 +100,9 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
   pdl_wait();  // the inputs are the predecessors' outputs
   pdl_trigger();
   if (threadIdx.x == 0) {
+    // the step's first kernel advances the clock: the previous step's kernels,
+    // its last readers, have completed, and this step's wait for this one
+    if (blockIdx.x == 0 && a.clock) *a.clock += 1;
     if (blockIdx.x < ntiles) issue(blockIdx.x, 0);
     if (blockIdx.x + gridDim.x < ntiles) issue(blockIdx.x + gridDim.x, 1);
   }

@@ -90,7 +90,7 @@ __global__ void k_record_field(const float* __restrict__ f, Sensor s, Clock clk,
 }
 
 __global__ void k_advance(int* t) {
-  pdl_wait();  // the step's kernels have read the clock
+  pdl_wait();  // the previous step's kernels have read the clock
   *t += 1;
 }
 
@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kThreads) k_fused_last(const __grid_constant__
   for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = tw_g[i];
   const int g = blockIdx.z;
   const int outer = blockIdx.y;
+  if (a.clock && threadIdx.x == 0 && blockIdx.x + outer + g == 0) *a.clock += 1;
   const long long off = (long long)outer * a.ostride;
   const float2* src = a.in[g] + off;
   const int c0 = blockIdx.x * tl;

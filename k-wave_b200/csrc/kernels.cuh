@@ -148,6 +148,7 @@ struct FusedArgs {
   int ncols;
   long long lstride, ostride;
   int tl;
+  int* clock;  // step clock this launch advances (nullptr: none)
 };
 
 struct UArgs {

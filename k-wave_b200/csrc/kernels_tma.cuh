@@ -52,6 +52,7 @@ struct FusedTmaArgs {
   // ncols - 1.  nrem: remainder tiles per input (0: none).
   CUtensorMap in_rem[3];
   int nrem, rem_y;
+  int* clock;  // step clock this launch advances (nullptr: none)
   int* err;
   TmaWaitArgs wait;
 };

@@ -674,9 +674,8 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
     p_buf.alloc(fb, st);
     ck(cudaMemsetAsync(p_buf.p, 0, fb, st), "memset");
   }
-  int one = 1;
   clock_buf.alloc(sizeof(int), st);
-  ck(cudaMemcpyAsync(clock_buf.p, &one, sizeof(int), cudaMemcpyHostToDevice, st), "clock");
+  ck(cudaMemsetAsync(clock_buf.p, 0, sizeof(int), st), "clock");  // each step's first kernel advances it
   clk.t = (const int*)clock_buf.p;
   clk.start = (int)opt.start_index;
 
@@ -919,7 +918,7 @@ void Session::col_pass(bool inv, const std::vector<int>& bufs, int z0, int nzs, 
 // The last-axis operator (z in 3D, y in 2D) over the whole volume: forward
 // transform, multiply by `fanout` operators per input, inverse transforms.
 void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& outs, const std::vector<SpecOp>& ops,
-                         int fanout, const std::vector<int>& dual, const float2* dual_tab) {
+                         int fanout, const std::vector<int>& dual, const float2* dual_tab, int* clock) {
   const int nin = (int)ins.size();
   const int nout = (int)outs.size();
   const int last = d.dim - 1;
@@ -953,6 +952,7 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
       for (int i = 0; i < nin; ++i) fa.in_rem[i] = map_zr[ins[i]];
     }
     fa.dim = d.dim;
+    fa.clock = clock;
     fa.ncols = d.nxh;
     fa.err = (int*)err_buf.p;
     fa.wait = tma_wait;
@@ -973,6 +973,7 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
     fa.lstride = (long long)d.nxp * (d.dim == 3 ? d.ny : 1);
     fa.ostride = d.nxp;
     fa.tl = col_tl[last];
+    fa.clock = clock;
     ck(launch_fused_last(fa, nin, d.dim == 3 ? d.ny : 1, plan[last], twd[last], T, d.dim, st), "fused_last");
   }
   ++launches_;
@@ -1001,14 +1002,16 @@ void Session::run_spectral(std::vector<int> ins, std::vector<int> outs, std::vec
 // a second output of kappa P.
 bool Session::grad_dual_in_y() const { return d.dim == 3 && use_tma[1]; }
 
-void Session::grad_pass() {
+// As the first kernel of a step it also advances the device clock.
+void Session::grad_pass(bool advance_clock) {
+  int* clock = advance_clock ? (int*)clock_buf.p : nullptr;
   if (d.dim == 3) {
     if (grad_dual_in_y())
-      fused_pass({0}, {1, 3}, {SpecOp{OP_KAPPA, 0}, SpecOp{OP_GRAD_POS, 2}}, 2);
+      fused_pass({0}, {1, 3}, {SpecOp{OP_KAPPA, 0}, SpecOp{OP_GRAD_POS, 2}}, 2, {}, nullptr, clock);
     else
-      fused_pass({0}, {1, 3}, {SpecOp{OP_KAPPA, 0}, SpecOp{OP_GRAD_POS, 2}}, 2, {2, -1}, T.ddk_pos[1]);
+      fused_pass({0}, {1, 3}, {SpecOp{OP_KAPPA, 0}, SpecOp{OP_GRAD_POS, 2}}, 2, {2, -1}, T.ddk_pos[1], clock);
   } else {
-    fused_pass({0}, {1, 2}, {SpecOp{OP_KAPPA, 0}, SpecOp{OP_GRAD_POS, 1}}, 2);
+    fused_pass({0}, {1, 2}, {SpecOp{OP_KAPPA, 0}, SpecOp{OP_GRAD_POS, 1}}, 2, {}, nullptr, clock);
   }
 }
 
@@ -1289,6 +1292,8 @@ void Session::build_sensor_lists(const uint64_t* lin, size_t n, std::vector<int>
 // t = 1 with an initial pressure (kspaceFirstOrder3D.m:1021-1035):
 // p = p0, rho_i = p0 / (dim c0^2), u_i = dt rho0_sg_inv grad_i(p0) / 2.
 void Session::enqueue_init() {
+  ck(launch_advance((int*)clock_buf.p, st), "advance");
+  ++launches_;
   const float* p0d = (const float*)p0_buf.p;
   ck(launch_record_field(p0d, row_sens_p(), clk, d.npts, st), "record p0");
   interp_points(0);
@@ -1300,7 +1305,7 @@ void Session::enqueue_init() {
   ck(launch_x_r2c(p0d, S[0], d, plan[0], twd[0], rowL, st), "x_r2c");
   ++launches_;
   col_pass(false, {0}, 0, d.nz);
-  grad_pass();
+  grad_pass(false);
   grad_col_inverse(0, d.nz);
   UArgs ua = u_args(S);
   ua.init = 1;
@@ -1359,17 +1364,22 @@ bool Session::graphable(uint64_t t) const {
   return true;
 }
 
+// `steps` steps from t captured as one graph.
+void Session::capture(uint64_t t, int steps, cudaGraph_t* g) {
+  ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
+  const uint64_t l0 = launches_;
+  for (int i = 0; i < steps; ++i) enqueue_step_body(t + i);
+  graph_launches = (launches_ - l0) / steps;
+  launches_ = l0;
+  ck(cudaStreamEndCapture(st, g), "end capture");
+}
+
 void Session::enqueue_step() {
   const uint64_t t = t_done + 1;
   if (graphable(t)) {
     if (!graph_exec) {
       cudaGraph_t g = nullptr;
-      ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-      const uint64_t l0 = launches_;
-      enqueue_step_body(t);
-      graph_launches = launches_ - l0;
-      launches_ = l0;
-      ck(cudaStreamEndCapture(st, &g), "end capture");
+      capture(t, 1, &g);
       graph = g;
       ++graph_gen;
       ck(cudaGraphInstantiate(&graph_exec, graph, 0), "graph instantiate");
@@ -1392,7 +1402,7 @@ void Session::enqueue_step_body(uint64_t t) {
     f12 = {1, 2};
     const bool last = (t == Nt);
     // (1) momentum: grad p -> u (kspaceFirstOrder3D.m:790-884)
-    grad_pass();
+    grad_pass(true);
     if (u_many_additive) {
       for (int a = 0; a < d.dim; ++a)
         if (udense[a].field && (int)t <= u_len[a]) {
@@ -1495,8 +1505,6 @@ void Session::enqueue_step_body(uint64_t t) {
       interp_points(0);
     }
   }
-  ck(launch_advance((int*)clock_buf.p, st), "advance");
-  ++launches_;
 }
 
 // corrected source field for "many" signals, using `work` as spectral scratch
@@ -1511,6 +1519,39 @@ void Session::corrected_source_into(float* out, const int* idx, const int* slot,
   launches_ += 4;
 }
 
+// Long advances replay kRunSteps steps per graph launch: consecutive graph
+// launches leave the device idle between them (no kernel of the next starts
+// before the last of the previous has ended and the launch is processed),
+// inside one graph a step's first kernel starts as the previous step's last
+// one ends.  Captured once an advance is long enough to pay for the capture.
+// False (nothing enqueued): fewer steps are left than a run takes, or one of
+// them cannot be replayed.
+bool Session::enqueue_run(uint64_t left) {
+  const uint64_t t = t_done + 1;
+  if (left < kRunSteps || (!run_exec && left < 8 * kRunSteps)) return false;
+  for (uint64_t i = 0; i < kRunSteps; ++i)
+    if (!graphable(t + i)) return false;
+  if (!run_exec) {
+    cudaGraph_t g = nullptr;
+    capture(t, kRunSteps, &g);
+    const cudaError_t e = cudaGraphInstantiate(&run_exec, g, 0);
+    cudaGraphDestroy(g);
+    ck(e, "graph instantiate");
+  }
+  ck(cudaGraphLaunch(run_exec, st), "graph launch");
+  launches_ += kRunSteps * graph_launches;
+  t_done += kRunSteps;
+  return true;
+}
+
+void Session::drop_graphs() {
+  if (graph_exec) cudaGraphExecDestroy(graph_exec);
+  if (run_exec) cudaGraphExecDestroy(run_exec);
+  if (graph) cudaGraphDestroy(graph);
+  graph_exec = run_exec = nullptr;
+  graph = nullptr;
+}
+
 void Session::advance(uint64_t n) {
   if (t_done + n > Nt) throw KwError(KW_ERR_INVALID_ARGUMENT, "advance beyond Nt");
   if (ring_rows) {  // rows recorded but not yet drained must still fit the ring
@@ -1519,7 +1560,12 @@ void Session::advance(uint64_t n) {
   }
   ck(cudaEventRecord(ev0, st), "event");
   const uint64_t l0 = launches_;
-  for (uint64_t i = 0; i < n; ++i) enqueue_step();
+  for (uint64_t i = 0; i < n;) {
+    if (enqueue_run(n - i))
+      i += kRunSteps;
+    else
+      enqueue_step(), ++i;
+  }
   last_launches = launches_ - l0;
   last_steps = n;
   ck(cudaEventRecord(ev1, st), "event");
@@ -1636,7 +1682,7 @@ void Session::restore_checkpoint(const std::string& path) {
       ck(cudaMemcpy(b->p, v.data(), b->bytes, cudaMemcpyHostToDevice), "checkpoint h2d");
     }
     t_done = t;
-    const int clock = (int)t + 1;  // the device clock holds the index of the next step
+    const int clock = (int)t;  // the device clock holds the index of the last step begun
     ck(cudaMemcpy(clock_buf.p, &clock, sizeof(int), cudaMemcpyHostToDevice), "clock");
   } catch (const h5::Error& e) {
     throw KwError(KW_ERR_IO, path + ": " + e.what());
@@ -1740,8 +1786,7 @@ void Session::read(kw_output* out) {
 
 Session::~Session() {
   if (st) cudaStreamSynchronize(st);
-  if (graph_exec) cudaGraphExecDestroy(graph_exec);
-  if (graph) cudaGraphDestroy(graph);
+  drop_graphs();
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (st2) {

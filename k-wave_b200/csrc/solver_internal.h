@@ -109,13 +109,16 @@ class Session {
   void col_pass(bool inv, const std::vector<int>& bufs, int z0, int nzs, int dual_field = -1, int dual_src = -1,
                 const float2* dual_tab = nullptr);
   void fused_pass(const std::vector<int>& ins, const std::vector<int>& outs, const std::vector<SpecOp>& ops,
-                  int fanout, const std::vector<int>& dual = {}, const float2* dual_tab = nullptr);
-  void grad_pass();
+                  int fanout, const std::vector<int>& dual = {}, const float2* dual_tab = nullptr,
+                  int* clock = nullptr);
+  void grad_pass(bool advance_clock);
   bool grad_dual_in_y() const;
   void grad_col_inverse(int z0, int nzs);
   Dims slab_dims(int z0, int nzs) const;
   void enqueue_init();
   void enqueue_step();
+  static constexpr uint64_t kRunSteps = 8;
+  bool enqueue_run(uint64_t left);
   void enqueue_step_body(uint64_t t);
   bool graphable(uint64_t t) const;
   UArgs u_args(float2* const* S);
@@ -142,6 +145,9 @@ class Session {
   bool use_graph = true;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  cudaGraphExec_t run_exec = nullptr;  // kRunSteps steps, for long advances
+  void capture(uint64_t t, int steps, cudaGraph_t* g);
+  void drop_graphs();
   uint64_t graph_launches = 0;
   uint64_t graph_gen = 0;  // captures so far (a batch rebuilds its parent graph when this changes)
   SpecTables T{};

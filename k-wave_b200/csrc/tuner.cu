@@ -206,10 +206,7 @@ void Session::set_schedule(const Schedule& s0) {
   cuda_ck(cudaStreamSynchronize(st), "sync");
   if (st2) cuda_ck(cudaStreamSynchronize(st2), "sync");
   // the captured step holds the old launch shapes
-  if (graph_exec) cuda_ck(cudaGraphExecDestroy(graph_exec), "cudaGraphExecDestroy");
-  if (graph) cuda_ck(cudaGraphDestroy(graph), "cudaGraphDestroy");
-  graph_exec = nullptr;
-  graph = nullptr;
+  drop_graphs();
   if (s.streams == 2 && !st2) {
     int lo = 0, hi = 0;
     cuda_ck(cudaDeviceGetStreamPriorityRange(&lo, &hi), "stream priority range");

@@ -1,0 +1,54 @@
+"""Long advances replay several steps per graph launch, short ones a single
+step, and steps that cannot be replayed run on their own: the same kernels on
+the same data each time, so every split of a run gives the same outputs bit for
+bit.  The device clock is advanced by each step's first kernel."""
+import numpy as np
+import pytest
+
+from helpers import case_2d_p0, case_3d_het, compare, oracle_outputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(inp, record, start, chunks):
+    from kwave import _lib
+
+    s = _lib.Session(inp, record, start)
+    try:
+        for n in chunks:
+            s.advance(n)
+        assert s.steps_done == sum(chunks)
+        return s.read()
+    finally:
+        s.close()
+
+
+def _cases():
+    yield case_2d_p0(n=(64, 48), nt=150, record=("p", "p_max", "p_rms", "u", "u_final"))  # step 1 is not replayed
+    yield case_3d_het(n=(40, 42, 45), nt=150, record=("p", "p_max", "p_rms", "u"))
+    yield case_3d_het(n=(40, 42, 45), nt=150, many=True, record=("p", "p_rms"))  # per-step corrected source
+    yield case_3d_het(n=(28, 36, 35), nt=150, record=("p", "p_rms"))  # runtime-plan engine
+
+
+@pytest.mark.parametrize("which", range(4))
+def test_every_split_of_a_run_gives_the_same_outputs(which):
+    inp, record, start, _ = list(_cases())[which]
+    whole = _run(inp, record, start, [150])
+    for chunks in ([1] * 150, [7, 64, 65, 1, 13], [149, 1], [63, 87]):
+        part = _run(inp, record, start, chunks)
+        for k in whole:
+            np.testing.assert_array_equal(part[k], whole[k], err_msg=f"{k} {chunks[:3]}")
+
+
+# (c_ref dt |k| / 2)^2 reaches (0.5 pi cfl)^2 dim: below 1 the operators take
+# the short sinc series, above it the long one
+@pytest.mark.parametrize("scale", [1.0, 1.2, 1.3, 2.0])
+def test_sinc_series_on_both_sides_of_the_rule(scale):
+    from kwave import _lib
+
+    inp, record, start, _ = case_3d_het(n=(48, 54, 56), nt=10, record=("p", "p_max", "p_rms", "u", "p_final"))
+    inp = dict(inp, dt=inp["dt"] * scale)
+    gpu = _lib.solve(inp, record=record, start_index=start)
+    errs = compare(gpu, oracle_outputs(inp, record, start, dtype=np.float64))
+    bad = {k: v for k, v in errs.items() if not v <= 1e-4}
+    assert errs and not bad, errs
