@@ -317,8 +317,9 @@ __device__ __forceinline__ void ct_last_st(const float2* buf, const float2* __re
   }
 }
 
-// The first stage with a caller-supplied loader: ld(l, pos) returns input
-// element pos of line l from wherever the caller keeps it (the row kernels
+// The first stage with a caller-supplied loader: ld(l, j, c, span) returns
+// input element j + c of line l, 0 <= j < span, c and span compile-time
+// constants once unrolled, from wherever the caller keeps it (the row kernels
 // build each packed line from two raw half-spectrum rows on the fly).  In
 // place like ct_stage: every input is loaded before the block barrier and
 // every output stored after it, so the inputs may alias the output buffer.
@@ -331,7 +332,7 @@ __device__ __forceinline__ void ct_stage0_ld(float2* buf, int l, int tid, L lay,
     const int j = tid + i * G::T;
     if (G::has(j)) {
 #pragma unroll
-      for (int r = 0; r < G::R; ++r) v[i][r] = ld(l, j + r * G::NR);
+      for (int r = 0; r < G::R; ++r) v[i][r] = ld(l, j, r * G::NR, G::NR);
       ct_butterfly<G, INV>(v[i], nullptr, j);  // first stage: no twiddles
     }
   }

@@ -167,23 +167,34 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
     };
     // prescaled: u already holds kappa * scale times the transform (GRAD)
     auto apply = [&](const OpEval& ev, float2 (&u)[M], bool prescaled = false) {
+      if constexpr (CLS == FC_GRAD) {
+        if (prescaled) {
 #pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const int p = tid + TPL * m;
-        const float k2 = kxy2 + kl2[p];
-        float f;
-        if constexpr (CLS == FC_GRAD) {
-          if (prescaled) {
-            u[m] = c_mul(u[m], ev.dline ? ev.dline[p] : ev.dconst);
-            continue;
+          for (int m = 0; m < M; ++m) u[m] = c_mul(u[m], ev.dline ? ev.dline[tid + TPL * m] : ev.dconst);
+        } else if (T.unit && ev.kappa) {  // every (cdt2 |k|)^2 <= 1: the short series
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            const int p = tid + TPL * m;
+            const float f = sinc_sq_unit(cdt2sq * (kxy2 + kl2[p])) * T.scale;
+            u[m] = c_mul(c_scale(u[m], f), ev.dline ? ev.dline[p] : ev.dconst);
           }
-          f = ev.kappa ? sinc_sq(cdt2sq * k2) * T.scale : T.scale;
-          u[m] = c_mul(c_scale(u[m], f), ev.dline ? ev.dline[p] : ev.dconst);
-        } else if constexpr (CLS == FC_NABLA) {
-          f = (k2 == 0.f) ? (ev.e == 0.f ? T.scale : 0.f) : exp2f(ev.e * log2f(k2)) * T.scale;
-          u[m] = c_scale(u[m], f);
         } else {
-          f = cos_sq(cdt2sq * k2) * T.scale;
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            const int p = tid + TPL * m;
+            const float f = ev.kappa ? sinc_sq(cdt2sq * (kxy2 + kl2[p])) * T.scale : T.scale;
+            u[m] = c_mul(c_scale(u[m], f), ev.dline ? ev.dline[p] : ev.dconst);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          const float k2 = kxy2 + kl2[tid + TPL * m];
+          float f;
+          if constexpr (CLS == FC_NABLA)
+            f = (k2 == 0.f) ? (ev.e == 0.f ? T.scale : 0.f) : exp2f(ev.e * log2f(k2)) * T.scale;
+          else
+            f = cos_sq(cdt2sq * k2) * T.scale;
           u[m] = c_scale(u[m], f);
         }
       }

@@ -574,19 +574,25 @@ __device__ __forceinline__ void drain_rows(uint64_t* bars, int from, int to, con
     for (int f = from; f < to; ++f) mbar_wait(&bars[f], 0, nullptr, wait_limit(w));
 }
 
-// Element n of packed line l, read from raw rows 2l and 2l + 1: the full
+// Element n = j + c of packed line l, read from raw rows 2l and 2l + 1: the full
 // spectrum of row 2l plus i times that of row 2l + 1, each from its half
 // spectrum (Hermitian), with the imaginary parts of the k = 0 and Nyquist
 // bins dropped, as load_c2r builds it.  `kmul` (optional) multiplies bin k.
+// c and span are compile-time constants (ct_stage0_ld), so which half of the
+// spectrum an element lies in, and whether it can be the k = 0 or the Nyquist
+// bin, is settled at compile time for nearly all of them.
 template <int NC>
 struct RawRows {
   const float2* raw;
   int nxp;
   int rows;
   const float2* kmul;
-  __device__ __forceinline__ float2 operator()(int l, int n) const {
-    const bool lo = 2 * n <= NC;
+  __device__ __forceinline__ float2 operator()(int l, int j, int c, int span) const {
+    const int n = j + c;
+    // from NC / 2 on the mirrored form holds (at NC / 2 itself both agree)
+    const bool lo = 2 * c >= NC ? false : (2 * (c + span - 1) <= NC ? true : 2 * n <= NC);
     const int k = lo ? n : NC - n;
+    const bool may_zero = c == 0, may_nyquist = 2 * c <= NC && 2 * (c + span - 1) >= NC;
     const int ra = 2 * l;
     float2 A = make_float2(0.f, 0.f), B = A;
     if (ra < rows) A = raw[ra * nxp + k];
@@ -596,7 +602,7 @@ struct RawRows {
       A = c_mul(A, m);
       B = c_mul(B, m);
     }
-    if (k == 0 || 2 * k == NC) {
+    if ((may_zero && n == 0) || (may_nyquist && 2 * n == NC)) {
       A.y = 0.f;
       B.y = 0.f;
     }
@@ -824,7 +830,7 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::MIN_BLOCK
   // every divergence component's spectrum rows are requested first (not on
   // axisymmetric grids, whose u_r / r spectrum is summed in as S[1] is read)
   __shared__ uint64_t rbar[3];
-  const bool bulk = RowBulk<NC, V>::OK && !a.S_rr;
+  const bool bulk = RowBulk<NC, V>::OK && (DIM == 3 || !a.S_rr);
   if constexpr (RowBulk<NC, V>::OK) {
     if (bulk && threadIdx.x == 0) {
       _Pragma("unroll") for (int f = 0; f < dim; ++f) mbar_init(&rbar[f], 1);
@@ -1294,7 +1300,7 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::EOS_BLOCK
 }
 
 // ---------------------------------------------------------------------------
-// plain x transforms (setup work, sources with k-space correction)
+// plain x transforms (setup work, sources with k-space correction), variant 0
 // ---------------------------------------------------------------------------
 template <int NC, int V>
 __global__ void __launch_bounds__(RTile<NC, V>::THREADS) k_x_r2c(const float* __restrict__ f, float2* S, Dims d,
@@ -1496,12 +1502,12 @@ void CtKernels<NC>::x_eos(const EosArgs& a, const Dims& d, const FFTPlan& plan, 
 template <int NC>
 void CtKernels<NC>::x_r2c(const float* f, float2* S, const Dims& d, const FFTPlan& plan, const float2* tw,
                           int L, cudaStream_t st) {
-  with_variant<NC>(d.v, [&](auto v) { x_r2c_t<NC, v.value>(f, S, d, plan, tw, L, st); });
+  x_r2c_t<NC, 0>(f, S, d, plan, tw, L, st);
 }
 template <int NC>
 void CtKernels<NC>::x_c2r(const float2* S, float* out, int acc, const Dims& d, const FFTPlan& plan,
                           const float2* tw, int L, cudaStream_t st) {
-  with_variant<NC>(d.v, [&](auto v) { x_c2r_t<NC, v.value>(S, out, acc, d, plan, tw, L, st); });
+  x_c2r_t<NC, 0>(S, out, acc, d, plan, tw, L, st);
 }
 
 }  // namespace kwb

@@ -542,6 +542,15 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
     T.shift_neg[2] = T.shift_neg[1];
   }
   T.cdt2 = (float)(c_ref * dt / 2.0);
+  {
+    double k2 = 0.0;
+    for (int a = 0; a < d.dim; ++a) {
+      double m = 0.0;
+      for (double k : kvec_fft_order(ns[a], dd[a])) m = std::max(m, k * k);
+      k2 += m;
+    }
+    T.unit = k2 * (double)T.cdt2 * (double)T.cdt2 <= 0.999 ? 1 : 0;
+  }
   T.scale = (float)(1.0 / (double)d.npts);
   T.ym2 = (float)(in->alpha_power - 2.0);
   T.ym1 = (float)(in->alpha_power - 1.0);
