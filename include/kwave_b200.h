@@ -307,9 +307,8 @@ void kw_batch_destroy(kw_batch* b);
  *
  * Launch schedule of the time step.  The y-inverse / row / y-forward chains
  * of a 3D step run whole or as z slabs, the slabs on one stream or
- * alternating between two, and the runtime-plan FFT kernels (lengths with a
- * factor 7, or outside 64..1024) transform a chosen number of lines per
- * block: these give bit-identical results.  The runtime-plan engine's radix
+ * alternating between two, and the runtime-plan FFT kernels (lengths outside
+ * 40..1024) transform a chosen number of lines per block: these give bit-identical results.  The runtime-plan engine's radix
  * order can be chosen too (0: radix 16 first, 1: odd radices first, 2: no
  * radix 16); another order rounds differently, within FP32 rounding.
  */

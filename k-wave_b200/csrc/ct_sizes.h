@@ -1,7 +1,8 @@
 // Transform lengths with compile-time FFT kernels: every 2^a 3^b 5^c length
-// from 64 to 1024 (61 lengths).  build.py generates one translation
-// unit per length (explicit instantiation of CtKernels<N>) and compiles them
-// in parallel; any other length runs on the runtime-plan engine.
+// from 64 to 1024 (61 lengths); further lengths are in ct_more_sizes.h.
+// build.py generates one translation unit per length (explicit instantiation
+// of CtKernels<N>) and compiles them in parallel; any other length runs on the
+// runtime-plan engine.
 #pragma once
 
 #define KWB_CT_SIZES(X) \

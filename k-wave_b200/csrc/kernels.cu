@@ -2,7 +2,7 @@
 // lookup table, the runtime-plan instantiation (NC = 0) and the small
 // elementwise kernels.  The FFT-carrying kernel templates are in
 // kernels_impl.cuh; each compile-time length is instantiated in its own
-// translation unit, generated by build.py from ct_sizes.h.
+// translation unit, generated by build.py from ct_sizes.h and ct_more_sizes.h.
 #include <algorithm>
 #include <cstdlib>
 

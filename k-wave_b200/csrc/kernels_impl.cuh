@@ -10,14 +10,15 @@
 // The x axis is always the first forward / last inverse transform and is
 // done by the row kernels (k_x_*), which fuse C2R -> elementwise physics ->
 // R2C so each field row is read and written once.  The y axis (3D) is a
-// column pass (k_col_fft) and the last axis (z in 3D, y in 2D) is done by
-// k_fused_last: forward, operator multiply, inverse, in one kernel.
+// column pass (col_tma.cuh; k_col_fft here without TMA) and the last axis (z
+// in 3D, y in 2D) forward transform, operator multiply and inverse in one
+// kernel (fused_tma.cuh; k_fused_last in kernels.cu without TMA).
 //
 // Every FFT-carrying kernel is a template on NC, the length of the axis it
-// transforms: NC > 0 selects the compile-time engine (fft_ct.cuh: in-place
-// register-staged stages, one shared-memory buffer per field, index math
-// folded to constants); NC == 0 is the runtime-plan engine for any other
-// 2^a 3^b 5^c length.
+// transforms, and V, its radix-plan variant: NC > 0 selects the compile-time
+// engine (fft_ct.cuh: in-place register-staged stages, one shared-memory
+// buffer per field, index math folded to constants); NC == 0 is the
+// runtime-plan engine for any other 2^a 3^b 5^c 7^d length.
 #pragma once
 #include <type_traits>
 

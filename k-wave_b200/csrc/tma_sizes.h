@@ -1,8 +1,8 @@
 // Transform lengths of the TMA-fed column passes (the y pass and the fused
-// last-axis operator): every 2^a 3^b 5^c length from 64 to 256 (a tensor
-// copy's box holds at most 256 elements along a dimension).  build.py
-// generates one translation unit per length for the fused operator
-// (fused_tma_N.cu, an explicit instantiation of fused_tma_cls<N>) and
+// last-axis operator) whose line is one segment of a tensor copy's box (at
+// most 256 elements along a dimension): every 2^a 3^b 5^c length from 64 to
+// 256.  Further lengths: tma_more_sizes.h.  build.py generates one translation
+// unit per length (tma_N.cu, an explicit instantiation of TmaKernels<N>) and
 // compiles them in parallel.
 #pragma once
 
