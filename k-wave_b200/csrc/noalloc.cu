@@ -103,8 +103,8 @@ __device__ __forceinline__ float sinc(float x) { return x == 0.f ? 1.f : sinf(x)
 // Phase 1: along y per group of tl kx columns: forward FFT, multiply by
 //          kappa and the two shifted derivatives, inverse FFTs into S[0], S[1].
 // Phase 2: C2R along x of S[c] into g[c] (blockIdx.y = component c).
-// The phases are launched with programmatic stream serialization: each builds
-// its twiddles while the one before ends (pdl_wait, tma.cuh).
+// Phases 1 and 2 are launched with programmatic stream serialization: each
+// builds its twiddles while the one before ends (pdl_wait, tma.cuh).
 __global__ void __launch_bounds__(THREADS) k_grad2d_noalloc(GradArgs a, int phase) {
   extern __shared__ float2 sm[];
   if (phase == 0) {
@@ -297,7 +297,9 @@ extern "C" int kw_kspace_gradient_noalloc(const float* d_f, float* d_gx, float* 
   const size_t row_smem = sizeof(float2) * (NX + 2 * row_layout_stride(NX));
   const size_t col_smem = sizeof(float2) * ((size_t)NY + 3ull * NY * a.tl);
   const unsigned row_pairs = (unsigned)((NY + 1) / 2);
-  e = launch_pdl(k_grad2d_noalloc, dim3(row_pairs), dim3(THREADS), row_smem, st, a, 0);
+  // the first launch follows whatever the caller's stream holds: an ordinary one
+  k_grad2d_noalloc<<<row_pairs, THREADS, row_smem, st>>>(a, 0);
+  e = cudaGetLastError();
   if (e == cudaSuccess)
     e = launch_pdl(k_grad2d_noalloc, dim3((unsigned)((a.nxh + a.tl - 1) / a.tl)), dim3(THREADS), col_smem, st, a, 1);
   if (e == cudaSuccess)

@@ -1528,36 +1528,10 @@ void Session::corrected_source_into(float* out, const int* idx, const int* slot,
   launches_ += 4;
 }
 
-// Long advances replay kRunSteps steps per graph launch: consecutive graph
-// launches leave the device idle between them (no kernel of the next starts
-// before the last of the previous has ended and the launch is processed),
-// inside one graph a step's first kernel starts as the previous step's last
-// one ends.  Captured once an advance is long enough to pay for the capture.
-// False (nothing enqueued): fewer steps are left than a run takes, or one of
-// them cannot be replayed.
-bool Session::enqueue_run(uint64_t left) {
-  const uint64_t t = t_done + 1;
-  if (left < kRunSteps || (!run_exec && left < 8 * kRunSteps)) return false;
-  for (uint64_t i = 0; i < kRunSteps; ++i)
-    if (!graphable(t + i)) return false;
-  if (!run_exec) {
-    cudaGraph_t g = nullptr;
-    capture(t, kRunSteps, &g);
-    const cudaError_t e = cudaGraphInstantiate(&run_exec, g, 0);
-    cudaGraphDestroy(g);
-    ck(e, "graph instantiate");
-  }
-  ck(cudaGraphLaunch(run_exec, st), "graph launch");
-  launches_ += kRunSteps * graph_launches;
-  t_done += kRunSteps;
-  return true;
-}
-
 void Session::drop_graphs() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
-  if (run_exec) cudaGraphExecDestroy(run_exec);
   if (graph) cudaGraphDestroy(graph);
-  graph_exec = run_exec = nullptr;
+  graph_exec = nullptr;
   graph = nullptr;
 }
 
@@ -1569,12 +1543,7 @@ void Session::advance(uint64_t n) {
   }
   ck(cudaEventRecord(ev0, st), "event");
   const uint64_t l0 = launches_;
-  for (uint64_t i = 0; i < n;) {
-    if (enqueue_run(n - i))
-      i += kRunSteps;
-    else
-      enqueue_step(), ++i;
-  }
+  for (uint64_t i = 0; i < n; ++i) enqueue_step();
   last_launches = launches_ - l0;
   last_steps = n;
   ck(cudaEventRecord(ev1, st), "event");

@@ -117,8 +117,6 @@ class Session {
   Dims slab_dims(int z0, int nzs) const;
   void enqueue_init();
   void enqueue_step();
-  static constexpr uint64_t kRunSteps = 8;
-  bool enqueue_run(uint64_t left);
   void enqueue_step_body(uint64_t t);
   bool graphable(uint64_t t) const;
   UArgs u_args(float2* const* S);
@@ -145,7 +143,6 @@ class Session {
   bool use_graph = true;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
-  cudaGraphExec_t run_exec = nullptr;  // kRunSteps steps, for long advances
   void capture(uint64_t t, int steps, cudaGraph_t* g);
   void drop_graphs();
   uint64_t graph_launches = 0;

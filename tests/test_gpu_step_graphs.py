@@ -1,5 +1,4 @@
-"""Long advances replay several steps per graph launch, short ones a single
-step, and steps that cannot be replayed run on their own: the same kernels on
+"""Steps are replayed as a graph, and those that cannot be run on their own: the same kernels on
 the same data each time, so every split of a run gives the same outputs bit for
 bit.  The device clock is advanced by each step's first kernel."""
 import numpy as np
