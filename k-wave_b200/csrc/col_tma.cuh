@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, ColBounds<NC, V>::MIN_B
     if (f == a.dual_field) {  // the derived field: the first stage reads its input times the axis factor
       const int id = ct_tid<NC>(tw), l = id % TL, tid = id / TL;
       const float2* tab = a.dual_tab;
-      ct_stage0_ld<NC, V, INV>(b, l, tid, lay, [&](int ll, int j, int c, int) { return c_mul(b[lay(ll, j + c)], __ldg(tab + j + c)); });
-      ct_stages<NC, V, 1, Ct<NC, V>::S, INV, false>(b, tw, l, tid, lay);
+      ct_stage0_ld<NC, V, INV>(b, tw, l, tid, lay, [&](int ll, int j, int c, int) { return c_mul(b[lay(ll, j + c)], __ldg(tab + j + c)); });
+      ct_stages<NC, V, 1, Ct<NC, V>::S, INV>(b, tw, l, tid, lay);
     } else {
       ct_fft<NC, V, INV, true, TL>(b, tw, lay);
     }

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 #include <stdexcept>
@@ -74,9 +75,10 @@ void fck(cudaError_t e, const char* what) {
 void column_pass(const kw_fft3d_plan& p, int axis, bool inv, float2* S, cudaStream_t st) {
   const Dims& d = p.d;
   const int n = axis == 1 ? d.ny : d.nz;
-  if (tma_supported(n)) {
+  if (d.v >= 0 && tma_supported(n)) {
     ColTmaArgs ca;
     std::memset(&ca, 0, sizeof(ca));
+    ca.v = d.v;
     if (!make_spec_map(&ca.map[0], S, d, axis, n, ca.v)) throw std::runtime_error("tensor map of the spectrum");
     ca.nfields = 1;
     ca.dual_field = ca.dual_src = -1;
@@ -94,6 +96,7 @@ void column_pass(const kw_fft3d_plan& p, int axis, bool inv, float2* S, cudaStre
     ca.lstride = axis == 1 ? d.nxp : (long long)d.nxp * d.ny;
     ca.ostride = axis == 1 ? (long long)d.nxp * d.ny : d.nxp;
     ca.tl = p.col_tl[axis];
+    ca.v = d.v;
     fck(launch_col_fft(inv, ca, 1, axis == 1 ? d.nz : d.ny, p.plan[axis], p.tw[axis], st), "column pass");
   }
 }
@@ -120,6 +123,8 @@ int kw_fft3d_create(uint64_t nx, uint64_t ny, uint64_t nz, kw_fft3d_plan** out, 
   d.npts = (long long)d.nx * d.nrows;
   d.row0 = 0;
   d.row1 = d.nrows;
+  const char* fp = std::getenv("KWAVE_B200_TEST_FFT_PLAN");  // test hook, as in a session
+  if (fp) d.v = std::max(-1, std::min(1, std::atoi(fp)));
   const int ns[3] = {d.nx, d.ny, d.nz};
   try {
     fck(cudaGetDevice(&p->device), "cudaGetDevice");

@@ -3,8 +3,8 @@
 // The solver's spectral work is a sequence of 1D transforms along one grid
 // axis at a time: a batch of "lines" (rows along x, or columns along y / z)
 // is staged in shared memory and transformed there with a mixed-radix
-// Stockham auto-sort FFT (radices 16, 8, 4, 2, 5, 3; grid edges of the form
-// 2^a 3^b 5^c up to 1024).  Each stage loads R points per butterfly into
+// Stockham auto-sort FFT (radices 16, 8, 4, 2, 7, 5, 3; grid edges of the form
+// 2^a 3^b 5^c 7^d up to 4096).  Each stage loads R points per butterfly into
 // registers, applies the inter-stage twiddles from a table built in FP64 on
 // the host, runs a register-resident radix-R codelet and writes the result
 // to the other half of a ping-pong buffer.
@@ -50,8 +50,23 @@ __host__ __device__ inline float2 c_sub(float2 a, float2 b) {
   return make_float2(a.x - b.x, a.y - b.y);
 #endif
 }
+// Sums of two products, here and in the codelets below, name the product that
+// is rounded before the fused multiply-add: left to the compiler, the choice
+// differs from kernel to kernel, and the same transform would round
+// differently in each.
 __host__ __device__ inline float2 c_mul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
+}
+// The product with a spectral operator.
+__host__ __device__ inline float2 c_op_mul(float2 a, float2 op) {
+  return make_float2(fmaf(a.x, op.x, -(a.y * op.y)), fmaf(a.y, op.x, a.x * op.y));
+}
+// The product with a twiddle w of the forward transform's table, conjugated
+// for the inverse.  OTHER: the forward form with the other product rounded.
+template <bool INV, bool OTHER = false>
+__host__ __device__ inline float2 c_twiddle(float2 a, float2 w) {
+  if (INV) return make_float2(fmaf(a.x, w.x, a.y * w.y), fmaf(a.y, w.x, -(a.x * w.y)));
+  return OTHER ? c_op_mul(a, w) : c_mul(a, w);
 }
 __host__ __device__ inline float2 c_scale(float2 a, float s) {
 #ifdef KWB_F32X2
@@ -107,10 +122,10 @@ __device__ __forceinline__ void dft5(float2* v) {
   const float s2 = 0.587785252292473129168705954639072769f;   // sin(4 pi / 5)
   float2 t1 = c_add(v[1], v[4]), t2 = c_add(v[2], v[3]);
   float2 t3 = c_sub(v[1], v[4]), t4 = c_sub(v[2], v[3]);
-  float2 a1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-  float2 a2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-  float2 b1 = make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
-  float2 b2 = make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
+  float2 a1 = make_float2(fmaf(c2, t2.x, fmaf(c1, t1.x, v[0].x)), fmaf(c2, t2.y, fmaf(c1, t1.y, v[0].y)));
+  float2 a2 = make_float2(fmaf(c1, t2.x, fmaf(c2, t1.x, v[0].x)), fmaf(c1, t2.y, fmaf(c2, t1.y, v[0].y)));
+  float2 b1 = make_float2(fmaf(s1, t3.x, s2 * t4.x), fmaf(s1, t3.y, s2 * t4.y));
+  float2 b2 = make_float2(fmaf(s2, t3.x, -(s1 * t4.x)), fmaf(s2, t3.y, -(s1 * t4.y)));
   v[0] = c_add(v[0], c_add(t1, t2));
   float2 r1 = c_rot<INV>(b1), r2 = c_rot<INV>(b2);
   v[1] = c_add(a1, r1);
@@ -138,10 +153,14 @@ __device__ __forceinline__ void dft7(float2* v) {
   v[0] = c_add(x0, c_add(t1, c_add(t2, t3)));
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float2 a = make_float2(x0.x + ca[k][0] * t1.x + ca[k][1] * t2.x + ca[k][2] * t3.x,
-                                 x0.y + ca[k][0] * t1.y + ca[k][1] * t2.y + ca[k][2] * t3.y);
-    const float2 b = make_float2(sb[k][0] * d1.x + sb[k][1] * d2.x + sb[k][2] * d3.x,
-                                 sb[k][0] * d1.y + sb[k][1] * d2.y + sb[k][2] * d3.y);
+    auto cosines = [&](float x, float u, float v, float w) {
+      return fmaf(ca[k][2], w, fmaf(ca[k][1], v, fmaf(ca[k][0], u, x)));
+    };
+    auto sines = [&](float u, float v, float w) {
+      return fmaf(sb[k][2], w, fmaf(sb[k][0], u, sb[k][1] * v));
+    };
+    const float2 a = make_float2(cosines(x0.x, t1.x, t2.x, t3.x), cosines(x0.y, t1.y, t2.y, t3.y));
+    const float2 b = make_float2(sines(d1.x, d2.x, d3.x), sines(d1.y, d2.y, d3.y));
     const float2 r = c_rot<INV>(b);
     v[k + 1] = c_add(a, r);
     v[6 - k] = c_sub(a, r);
@@ -173,6 +192,16 @@ __device__ __forceinline__ void dft8(float2* v) {
   v[7] = c_sub(e3, w3);
 }
 
+// o W16^k = o exp(-+ i k pi / 8), k = 0 .. 7, from w = (cos, sin) of k pi / 8.
+// Which product of each sum is rounded first is as the compiler once chose for
+// these constants, kept so that results stay what they were.
+template <bool INV>
+__device__ __forceinline__ float2 w16_mul(float2 o, float2 w, int k) {
+  if (INV) return make_float2(fmaf(o.x, w.x, -(o.y * w.y)), fmaf(o.x, w.y, o.y * w.x));
+  return make_float2(k == 6 ? fmaf(o.y, w.y, o.x * w.x) : fmaf(o.x, w.x, o.y * w.y),
+                     k == 2 ? fmaf(o.x, -w.y, o.y * w.x) : fmaf(o.y, w.x, -(o.x * w.y)));
+}
+
 template <bool INV>
 __device__ __forceinline__ void dft16(float2* v) {
   // cos / sin of k*pi/8
@@ -187,87 +216,13 @@ __device__ __forceinline__ void dft16(float2* v) {
   }
   dft8<INV>(e);
   dft8<INV>(o);
-  // W16^k = exp(-+ i k pi / 8); k = 0 is 1, k = 4 a quarter turn, k = 2 and 6 diagonals
   const float wc[8] = {1.f, c1, r, s1, 0.f, -s1, -r, -c1};
   const float ws[8] = {0.f, s1, r, c1, 1.f, c1, r, s1};
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    float2 t;
-    if (k == 0) {
-      t = o[k];
-    } else if (k == 4) {
-      t = c_rot<INV>(o[k]);
-    } else if (k == 2) {
-      t = INV ? make_float2(r * (o[k].x - o[k].y), r * (o[k].x + o[k].y))
-              : make_float2(r * (o[k].x + o[k].y), r * (o[k].y - o[k].x));
-    } else if (k == 6) {
-      t = INV ? make_float2(-r * (o[k].x + o[k].y), r * (o[k].x - o[k].y))
-              : make_float2(r * (o[k].y - o[k].x), -r * (o[k].x + o[k].y));
-    } else {
-      t = c_mul(o[k], make_float2(wc[k], INV ? ws[k] : -ws[k]));
-    }
+    const float2 t = k == 0 ? o[k] : (k == 4 ? c_rot<INV>(o[k]) : w16_mul<INV>(o[k], make_float2(wc[k], ws[k]), k));
     v[k] = c_add(e[k], t);
     v[k + 8] = c_sub(e[k], t);
-  }
-}
-
-template <int R, bool INV>
-__device__ __forceinline__ void dft(float2* v);
-
-// R = A B with A and B coprime (6, 10, 12, 14, 15): the prime-factor form
-// (Good 1958), A-point and B-point transforms with no twiddles between them.
-// Input n = (B n1 + A n2) mod R; output k = (B b k1 + A a k2) mod R with
-// b = B^-1 mod A and a = A^-1 mod B.
-__host__ __device__ constexpr int inv_mod(int x, int m) {
-  for (int i = 1; i < m; ++i)
-    if (x % m * i % m == 1) return i;
-  return 1;
-}
-template <int A, int B, bool INV>
-__device__ __forceinline__ void dft_pfa(float2* v) {
-  constexpr int R = A * B, eb = B * inv_mod(B, A), ea = A * inv_mod(A, B);
-  float2 t[B][A];
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) {
-#pragma unroll
-    for (int n1 = 0; n1 < A; ++n1) t[n2][n1] = v[(B * n1 + A * n2) % R];
-    dft<A, INV>(t[n2]);
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < A; ++k1) {
-    float2 b[B];
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) b[n2] = t[n2][k1];
-    dft<B, INV>(b);
-#pragma unroll
-    for (int k2 = 0; k2 < B; ++k2) v[(eb * k1 + ea * k2) % R] = b[k2];
-  }
-}
-
-// 9-point: 3 x 3 with W9^(n2 k1) between the two layers.
-template <bool INV>
-__device__ __forceinline__ void dft9(float2* v) {
-  // cos / sin of 2 pi k / 9, k = 1, 2, 4
-  const float c[3] = {0.766044443118978035f, 0.173648177666930349f, -0.939692620785908384f};
-  const float s[3] = {0.642787609686539326f, 0.984807753012208059f, 0.342020143325668733f};
-  float2 t[3][3];
-#pragma unroll
-  for (int n2 = 0; n2 < 3; ++n2) {
-#pragma unroll
-    for (int n1 = 0; n1 < 3; ++n1) t[n2][n1] = v[3 * n1 + n2];
-    dft3<INV>(t[n2]);
-  }
-  auto w = [&](float2 a, int i) { return c_mul(a, make_float2(c[i], INV ? s[i] : -s[i])); };
-  t[1][1] = w(t[1][1], 0);
-  t[1][2] = w(t[1][2], 1);
-  t[2][1] = w(t[2][1], 1);
-  t[2][2] = w(t[2][2], 2);
-#pragma unroll
-  for (int k1 = 0; k1 < 3; ++k1) {
-    float2 b[3] = {t[0][k1], t[1][k1], t[2][k1]};
-    dft3<INV>(b);
-#pragma unroll
-    for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = b[k2];
   }
 }
 
@@ -285,18 +240,6 @@ __device__ __forceinline__ void dft(float2* v) {
     dft7<INV>(v);
   } else if constexpr (R == 8) {
     dft8<INV>(v);
-  } else if constexpr (R == 9) {
-    dft9<INV>(v);
-  } else if constexpr (R == 6) {
-    dft_pfa<2, 3, INV>(v);
-  } else if constexpr (R == 10) {
-    dft_pfa<2, 5, INV>(v);
-  } else if constexpr (R == 12) {
-    dft_pfa<4, 3, INV>(v);
-  } else if constexpr (R == 14) {
-    dft_pfa<2, 7, INV>(v);
-  } else if constexpr (R == 15) {
-    dft_pfa<3, 5, INV>(v);
   } else if constexpr (R == 16) {
     dft16<INV>(v);
   }
@@ -341,9 +284,7 @@ __device__ __forceinline__ void fft_stage(const float2* __restrict__ src, float2
     if (ns > 1) {
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        float2 w = tw[k * r * twstep];
-        if (INV) w.y = -w.y;
-        v[r] = c_mul(v[r], w);
+        v[r] = c_twiddle<INV>(v[r], tw[k * r * twstep]);
       }
     }
     dft<R, INV>(v);

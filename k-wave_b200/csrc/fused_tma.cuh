@@ -10,10 +10,16 @@ namespace kwb {
 // only that operator's arithmetic in the kernel body.
 enum FusedClass { FC_GRAD = 0, FC_NABLA = 1, FC_SRCK = 2 };
 
+// The operations an operator is evaluated in, and so its rounding: from |k|^2
+// (no square root) for the 2^a 3^b 5^c lengths from 64 to 256, whose results
+// have always been rounded so; from |k|, the very operations of eval_op, for
+// the others, so that they get the same bits here and in k_fused_last.
+template <int N>
+constexpr bool kOpFromK = N < 64 || N > 256 || N % 7 == 0;
+
 // Blocks per SM the register budget is sized for: about 768 threads for the
 // single-output pass, 512 otherwise and where a stage holds more than 16
-// elements a thread or a radix is a multiple of 7 (180 = 15 x 12 spilled
-// 0.26 KB a thread at 768).
+// elements a thread or a radix is 7, which spill at 768.
 template <int NC, int V, int MODE>
 struct FusedBounds {
   static constexpr int TH = TTile<NC, V>::THREADS;
@@ -109,7 +115,8 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
   const CtCol<TL> lay{};
   const float cdt2sq = T.cdt2 * T.cdt2;
   constexpr int TPL = TH / TL;  // threads per line
-  constexpr int M = CtHandoff<NC, V>::M;
+  using HO = CtHandoff<NC, V>;
+  constexpr int M = HO::M;
   static_assert(TPL == Ct<NC, V>::T, "one line per group of T threads");
   bool aborted = false;
   int it = 0;
@@ -161,43 +168,38 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
           }
         }
       } else if constexpr (CLS == FC_NABLA) {
-        ev.e = 0.5f * ((op.kind == OP_NABLA1) ? T.ym2 : T.ym1);  // |k|^y = (|k|^2)^(y/2)
+        ev.e = (op.kind == OP_NABLA1) ? T.ym2 : T.ym1;
       }
       return ev;
     };
-    // prescaled: u already holds kappa * scale times the transform (GRAD)
-    auto apply = [&](const OpEval& ev, float2 (&u)[M], bool prescaled = false) {
+    // the operator of element p of the line on u; prescaled: u already holds
+    // kappa * scale times the transform (GRAD)
+    auto apply1 = [&](const OpEval& ev, float2 u, int p, bool prescaled) -> float2 {
+      const float k2 = kxy2 + kl2[p];
       if constexpr (CLS == FC_GRAD) {
-        if (prescaled) {
-#pragma unroll
-          for (int m = 0; m < M; ++m) u[m] = c_mul(u[m], ev.dline ? ev.dline[tid + TPL * m] : ev.dconst);
-        } else if (T.unit && ev.kappa) {  // every (cdt2 |k|)^2 <= 1: the short series
-#pragma unroll
-          for (int m = 0; m < M; ++m) {
-            const int p = tid + TPL * m;
-            const float f = sinc_sq_unit(cdt2sq * (kxy2 + kl2[p])) * T.scale;
-            u[m] = c_mul(c_scale(u[m], f), ev.dline ? ev.dline[p] : ev.dconst);
-          }
-        } else {
-#pragma unroll
-          for (int m = 0; m < M; ++m) {
-            const int p = tid + TPL * m;
-            const float f = ev.kappa ? sinc_sq(cdt2sq * (kxy2 + kl2[p])) * T.scale : T.scale;
-            u[m] = c_mul(c_scale(u[m], f), ev.dline ? ev.dline[p] : ev.dconst);
-          }
+        const float2 d = ev.dline ? ev.dline[p] : ev.dconst;
+        if constexpr (kOpFromK<NC>) {
+          const float f = ev.kappa ? sinc_series(T.cdt2 * sqrtf(k2)) * T.scale : T.scale;
+          return c_op_mul(u, make_float2(d.x * f, d.y * f));
         }
+        if (prescaled) return c_op_mul(u, d);
+        const float f = ev.kappa ? sinc_sq(cdt2sq * k2) * T.scale : T.scale;
+        return c_op_mul(c_scale(u, f), d);
       } else {
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const float k2 = kxy2 + kl2[tid + TPL * m];
-          float f;
-          if constexpr (CLS == FC_NABLA)
-            f = (k2 == 0.f) ? (ev.e == 0.f ? T.scale : 0.f) : exp2f(ev.e * log2f(k2)) * T.scale;
-          else
-            f = cos_sq(cdt2sq * k2) * T.scale;
-          u[m] = c_scale(u[m], f);
+        float f;
+        if constexpr (CLS == FC_NABLA) {  // |k|^y = (|k|^2)^(y/2)
+          const float k = kOpFromK<NC> ? sqrtf(k2) : k2, e = kOpFromK<NC> ? ev.e : 0.5f * ev.e;
+          f = (k == 0.f) ? (e == 0.f ? T.scale : 0.f) : exp2f(e * log2f(k)) * T.scale;
+        } else {
+          f = (kOpFromK<NC> ? cos_series(T.cdt2 * sqrtf(k2)) : cos_sq(cdt2sq * k2)) * T.scale;
         }
+        return c_scale(u, f);
       }
+    };
+    auto apply = [&](const OpEval& ev, float2 (&u)[M], bool prescaled = false) {
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        if (HO::has(tid, m)) u[m] = apply1(ev, u[m], HO::pos(tid, m), prescaled);
     };
     // inverse last stage, straight from W to the output (and the optional
     // second output scaled by a factor constant along the line)
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
           if (dst2) dst2[pos * a.lstride] = c_mul(v, dsc);
         }
       };
-      ct_last_st<NC, V, true, false>(src, tw, l, tid, lay, st_g);
+      ct_last_st<NC, V, true>(src, tw, l, tid, lay, st_g);
       fence_async_smem();  // the reads of src come before a TMA refill of it
       __syncthreads();     // src is reused by the next inverse
     };
@@ -232,26 +234,35 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
     }
     if (threadIdx.x == 0) inflight &= ~(1u << s);
     float2 u[M];
-    ct_stages<NC, V, 0, S - 1, false, true>(F, tw, l, tid, lay);
-    ct_fwd_last_to_regs<NC, V>(F, tw, l, tid, lay, u);
+    auto load_u = [&]() {  // the inverse transform's first inputs
+#pragma unroll
+      for (int m = 0; m < M; ++m)
+        if (HO::has(tid, m)) u[m] = F[lay(l, HO::pos(tid, m))];
+    };
     if constexpr (MODE == 1) {
       // operator and inverse first stage in registers, the latter's outputs
       // back into F once every thread has read its inputs; inverse last
       // stage to the output; then F takes the tile two ahead
+      constexpr bool OTHER = NC == 64 || NC == 128 || NC == 256;  // as their results have always been rounded
+      if constexpr (HO::DIRECT) {
+        ct_stages<NC, V, 0, S - 1, false, OTHER>(F, tw, l, tid, lay);
+        ct_fwd_last_to_regs<NC, V, OTHER>(F, tw, l, tid, lay, u);
+      } else {
+        ct_stages<NC, V, 0, S, false, OTHER>(F, tw, l, tid, lay);
+        load_u();
+      }
       apply(setup(0), u);
       __syncthreads();
-      ct_inv_first_from_regs<NC, V>(u, F, l, tid, lay);
+      ct_inv_first_from_regs<NC, V>(u, tw, F, l, tid, lay);
       __syncthreads();
-      ct_stages<NC, V, 1, S - 1, true, false>(F, tw, l, tid, lay);
+      ct_stages<NC, V, 1, S - 1, true>(F, tw, l, tid, lay);
       finish(0, F);
       refill();
     } else {
-      // several outputs of one input: the forward transform is kept in F, each
-      // thread's own positions; each output is read from it, multiplied in
+      // several outputs of one input: the forward transform is kept in F; each
+      // output's first inverse inputs are read from it, multiplied in
       // registers and given the inverse first stage on the way to W
-      __syncthreads();
-#pragma unroll
-      for (int m = 0; m < M; ++m) F[lay(l, tid + TPL * m)] = u[m];
+      ct_stages<NC, V, 0, S, false>(F, tw, l, tid, lay);
       // a first output of kappa alone (the gradient pass: kappa P, then kappa
       // P times the axis derivative) leaves kappa * scale * F in F, so the
       // later outputs carrying kappa skip its evaluation (c_mul by 1 + 0i is
@@ -259,22 +270,22 @@ __global__ void __launch_bounds__(TTile<NC, V>::THREADS, FusedBounds<NC, V, MODE
       bool kf = false;
 #pragma unroll 1
       for (int q = 0; q < a.fanout; ++q) {
-#pragma unroll
-        for (int m = 0; m < M; ++m) u[m] = F[lay(l, tid + TPL * m)];
+        load_u();
         const OpEval ev = setup(q);
         apply(ev, u, kf && ev.kappa);
-        if constexpr (CLS == FC_GRAD) {
+        if constexpr (CLS == FC_GRAD && !kOpFromK<NC>) {
           if (q == 0 && a.fanout > 1 && a.op[g * a.fanout].kind == OP_KAPPA) {
 #pragma unroll
-            for (int m = 0; m < M; ++m) F[lay(l, tid + TPL * m)] = u[m];  // this thread's own positions
+            for (int m = 0; m < M; ++m)
+              if (HO::has(tid, m)) F[lay(l, HO::pos(tid, m))] = u[m];  // no other thread reads them
             kf = true;
           }
         }
-        ct_inv_first_from_regs<NC, V>(u, W, l, tid, lay);
+        ct_inv_first_from_regs<NC, V>(u, tw, W, l, tid, lay);
         if (q + 1 == a.fanout) fence_async_smem();
         __syncthreads();
         if (q + 1 == a.fanout) refill();
-        ct_stages<NC, V, 1, S - 1, true, false>(W, tw, l, tid, lay);
+        ct_stages<NC, V, 1, S - 1, true>(W, tw, l, tid, lay);
         finish(q, W);
       }
     }

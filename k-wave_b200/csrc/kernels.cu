@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kThreads) k_fused_last(const __grid_constant__
       if (c >= a.ncols) c = 0;
       const int iy = (dim == 3) ? outer : p;
       const int iz = (dim == 3) ? p : 0;
-      W1[i] = c_mul(F[i], eval_op(op, T, dim, c, iy, iz));
+      W1[i] = c_op_mul(F[i], eval_op(op, T, dim, c, iy, iz));
     }
     __syncthreads();
     float2* R = fft_lines<true, true>(W1, C, tw, plan, tl, lay);
@@ -192,9 +192,11 @@ const CtEntry kRuntime = {0,
                           &CtKernels<0>::threads_per_line};
 
 // the kernels of transform length n: compile-time if listed, else runtime
-const CtEntry& kernels_for(int n) {
-  for (const CtEntry& e : kCtTable)
-    if (e.n == n) return e;
+// (plan variant v < 0: runtime)
+const CtEntry& kernels_for(int n, int v = 0) {
+  if (v >= 0)
+    for (const CtEntry& e : kCtTable)
+      if (e.n == n) return e;
   return kRuntime;
 }
 
@@ -216,7 +218,7 @@ int plan_variant(int n, long long lines) {
 
 cudaError_t launch_col_fft(bool inv, const ColArgs& a, int nfields, long long nouter, const FFTPlan& plan,
                            const float2* tw, cudaStream_t st) {
-  kernels_for(plan.n).col_fft(inv, a, nfields, nouter, plan, tw, st);
+  kernels_for(plan.n, a.v).col_fft(inv, a, nfields, nouter, plan, tw, st);
   return cudaGetLastError();
 }
 
@@ -231,31 +233,31 @@ cudaError_t launch_fused_last(const FusedArgs& a, int ninputs, long long nouter,
 
 cudaError_t launch_x_u(const UArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                        cudaStream_t st) {
-  kernels_for(d.nx).x_u(a, d, plan, tw, L, st);
+  kernels_for(d.nx, d.v).x_u(a, d, plan, tw, L, st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_x_rho(const RhoArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                          cudaStream_t st) {
-  kernels_for(d.nx).x_rho(a, d, plan, tw, L, st);
+  kernels_for(d.nx, d.v).x_rho(a, d, plan, tw, L, st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_x_eos(const EosArgs& a, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                          cudaStream_t st) {
-  kernels_for(d.nx).x_eos(a, d, plan, tw, L, st);
+  kernels_for(d.nx, d.v).x_eos(a, d, plan, tw, L, st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_x_r2c(const float* f, float2* S, const Dims& d, const FFTPlan& plan, const float2* tw, int L,
                          cudaStream_t st) {
-  kernels_for(d.nx).x_r2c(f, S, d, plan, tw, L, st);
+  kernels_for(d.nx, d.v).x_r2c(f, S, d, plan, tw, L, st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_x_c2r(const float2* S, float* out, int accumulate, const Dims& d, const FFTPlan& plan,
                          const float2* tw, int L, cudaStream_t st) {
-  kernels_for(d.nx).x_c2r(S, out, accumulate, d, plan, tw, L, st);
+  kernels_for(d.nx, d.v).x_c2r(S, out, accumulate, d, plan, tw, L, st);
   return cudaGetLastError();
 }
 

@@ -48,7 +48,6 @@ struct SpecTables {
   const float2* ddk_neg[3];  // i k exp(-i k d / 2)
   const float2* shift_neg[3];  // exp(-i k d / 2) (kspaceFirstOrder_createStorageVariables.m)
   float cdt2;                // c_ref * dt / 2
-  int unit;                  // (cdt2 |k|)^2 <= 1 at every bin
   float ym2, ym1;            // alpha_power - 2, alpha_power - 1
   float scale;               // 1 / (nx ny nz): the inverse-FFT normalisation
 };

@@ -465,6 +465,17 @@ __device__ __forceinline__ void row_unit(int u, int& q, int& x) {
   }
 }
 
+// pm * v + damp * s, the source's product rounded first (FIRST) or the other.
+// Which one is part of a length's results: the 4-wide epilogue of the lengths
+// from 64 without a factor 7 rounds the source's, the other paths, and with
+// them the lengths that once ran only those, the other.
+template <bool FIRST>
+__device__ __forceinline__ float add_source(float pm, float v, float damp, float s) {
+  return FIRST ? fmaf(pm, v, damp * s) : fmaf(damp, s, pm * v);
+}
+template <int NC>
+constexpr bool kSourceFirst = NC >= 64 && NC % 7 != 0;
+
 template <int NC, int V>
 __device__ __forceinline__ int row_lines(int L) {
   return NC > 0 ? RTile<NC, V>::LINES : L;
@@ -722,7 +733,7 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, NC == 256 ? (LEAN ? 8 :
           un = a.dt * rvv[j] * g / 2.f;
         else
           un = pmv[j] * (pmv[j] * uov[j] - a.dt * rvv[j] * g);
-        if (dense_on) un = un + damp * svv[j];
+        if (dense_on) un = fmaf(damp, svv[j], un);
         set_comp(G, lay, q, x + j, un);
       }
     }
@@ -747,7 +758,7 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, NC == 256 ? (LEAN ? 8 :
         un = a.dt * rv * g / 2.f;
       else
         un = pm * (pm * u[gi] - a.dt * rv * g);
-      if (dense_on) un = un + damp * __ldg(ds.field + gi);
+      if (dense_on) un = fmaf(damp, __ldg(ds.field + gi), un);
       set_comp(G, lay, q, x, un);
     }
   }
@@ -988,8 +999,8 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::MIN_BLOCK
           }
           _Pragma("unroll") for (int f = 0; f < dim; ++f) {
             const float pm = c(pm4[f]);
-            rn[f][j] = pm * (pm * rold[f] - a.dt * rpr * du[f]);
-            if (dense_on) rn[f][j] = rn[f][j] + damp * c(ds4);
+            const float v = pm * rold[f] - a.dt * rpr * du[f];
+            rn[f][j] = dense_on ? add_source<kSourceFirst<NC>>(pm, v, damp, c(ds4)) : pm * v;
           }
           rsum = rn[0][j] + rn[1][j];
           if (dim == 3) rsum += rn[2][j];
@@ -1088,8 +1099,8 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::MIN_BLOCK
           const int coord[3] = {x, y, z};
           _Pragma("unroll") for (int f = 0; f < dim; ++f) {
             const float pm = __ldg(a.pml[f] + coord[f]);
-            rnew[f] = pm * (pm * rold[f] - a.dt * rpr * du[f]);
-            if (dense_on) rnew[f] = rnew[f] + damp * __ldg(a.dsrc.field + gi);
+            const float v = pm * rold[f] - a.dt * rpr * du[f];
+            rnew[f] = dense_on ? add_source<false>(pm, v, damp, __ldg(a.dsrc.field + gi)) : pm * v;
             a.rho[f][gi] = rnew[f];
           }
           if (sp) continue;

@@ -470,6 +470,10 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
   plan_v[0] = d.v = plan_variant(d.nx, (d.nrows + 1) / 2);
   plan_v[1] = plan_variant(d.ny, (long long)d.nxh * d.nz);
   plan_v[2] = d.dim == 3 ? plan_variant(d.nz, (long long)d.nxh * d.ny) : 0;
+  // test hook: one variant on every axis, -1 the runtime-plan engine (the same bits)
+  const char* fp = std::getenv("KWAVE_B200_TEST_FFT_PLAN");
+  if (fp) plan_v[0] = plan_v[1] = plan_v[2] = d.v = std::max(-1, std::min(1, std::atoi(fp)));
+  const bool runtime_fft = plan_v[0] < 0;
 
   // ----- operator tables -----
   const double dd[3] = {in->dx, in->dy, in->dz};
@@ -542,15 +546,6 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
     T.shift_neg[2] = T.shift_neg[1];
   }
   T.cdt2 = (float)(c_ref * dt / 2.0);
-  {
-    double k2 = 0.0;
-    for (int a = 0; a < d.dim; ++a) {
-      double m = 0.0;
-      for (double k : kvec_fft_order(ns[a], dd[a])) m = std::max(m, k * k);
-      k2 += m;
-    }
-    T.unit = k2 * (double)T.cdt2 * (double)T.cdt2 <= 0.999 ? 1 : 0;
-  }
   T.scale = (float)(1.0 / (double)d.npts);
   T.ym2 = (float)(in->alpha_power - 2.0);
   T.ym1 = (float)(in->alpha_power - 1.0);
@@ -654,7 +649,7 @@ void Session::setup(const kw_input* in, const kw_options* o, bool allow_ring) {
   use_graph = !(no_graph && no_graph[0] == '1');
   // TMA-fed column passes for the compile-time lengths they support
   const char* no_tma = std::getenv("KWAVE_B200_NO_TMA");
-  const bool tma_ok = !(no_tma && no_tma[0] == '1');
+  const bool tma_ok = !(no_tma && no_tma[0] == '1') && !runtime_fft;
   // the TMA kernels' wait limit (microseconds; default 2 s) and the failure-
   // detection test's hook (a tile whose load is never issued)
   if (const char* w = std::getenv("KWAVE_B200_TMA_WAIT_US")) {

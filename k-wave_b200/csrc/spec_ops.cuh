@@ -28,18 +28,6 @@ __device__ __forceinline__ float sinc_sq(float u) {
   return s;
 }
 
-// The same for u <= 1, where six terms reach FP32 rounding (the next one is
-// below 1 / 13! = 1.6e-10).
-__device__ __forceinline__ float sinc_sq_unit(float u) {
-  float s = -2.5052108385441720e-08f;           // -1/11!
-  s = fmaf(s, u, 2.7557319223985893e-06f);      //  1/9!
-  s = fmaf(s, u, -1.9841269841269841e-04f);     // -1/7!
-  s = fmaf(s, u, 8.3333333333333333e-03f);      //  1/5!
-  s = fmaf(s, u, -1.6666666666666667e-01f);     // -1/3!
-  s = fmaf(s, u, 1.0f);
-  return s;
-}
-
 __device__ __forceinline__ float cos_sq(float u) {
   if (u > 9.8696044f) return cosf(sqrtf(u));
   float s = 4.1103176233121648e-19f;            //  1/20!
