@@ -285,7 +285,9 @@ struct CtRow {
   static constexpr int stride() {
     int ls = N + ((N - 1) >> SH);
     if (N % 4 == 0 && ls < N + 4) ls = N + 4;  // two raw half-spectrum rows fit one line (RowBulk)
-    while (ls % 16 != Ct<N, V>::T % 16) ++ls;
+    // one line of an odd number of threads: an even stride, for the bulk copies' 16 bytes
+    const int t = Ct<N, V>::T, even = N % 4 == 0 && t % 2 == 1 && ct_row_lines(t, V) == 1;
+    while (ls % 16 != (t + even) % 16) ++ls;
     return ls;
   }
   static constexpr int LS = stride();
