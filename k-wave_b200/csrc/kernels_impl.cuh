@@ -454,7 +454,7 @@ __device__ __forceinline__ float src_value(const SparseSource& s, const float* s
 // ms per 256^3 step.)
 template <int NC, int V>
 __device__ __forceinline__ void row_unit(int u, int& q, int& x) {
-  constexpr int Q = NC / 4;
+  constexpr int Q = NC > 0 ? NC / 4 : 1;
   if constexpr (CtRow<NC, V>::SH == 4) {
     q = u / Q;
     x = 4 * (u - q * Q);
@@ -1314,18 +1314,18 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS, RTile<NC, V>::EOS_BLOCK
 // ---------------------------------------------------------------------------
 // plain x transforms (setup work, sources with k-space correction), variant 0
 // ---------------------------------------------------------------------------
-template <int NC, int V>
-__global__ void __launch_bounds__(RTile<NC, V>::THREADS) k_x_r2c(const float* __restrict__ f, float2* S, Dims d,
+template <int NC>
+__global__ void __launch_bounds__(RTile<NC, 0>::THREADS) k_x_r2c(const float* __restrict__ f, float2* S, Dims d,
                                                              const __grid_constant__ FFTPlan plan,
                                                              const float2* __restrict__ tw_g, int Lrt) {
   extern __shared__ __align__(16) float2 sm[];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC, V>(Lrt);
-  const auto lay = row_lay<NC, V>(nx);
+  const int L = row_lines<NC, 0>(Lrt);
+  const auto lay = row_lay<NC, 0>(nx);
   float2* tw = sm;
   float2* B0 = sm + nx;
-  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, V>(nx);
+  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, 0>(nx);
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   const int total = 2 * L * nx;
@@ -1335,29 +1335,29 @@ __global__ void __launch_bounds__(RTile<NC, V>::THREADS) k_x_r2c(const float* __
     set_comp(B0, lay, q, x, row < d.row1 ? f[row * nx + x] : 0.f);
   }
   __syncthreads();
-  float2* F = row_fft<NC, V, false>(B0, B1, tw, plan, L, lay);
+  float2* F = row_fft<NC, 0, false>(B0, B1, tw, plan, L, lay);
   store_r2c<NC>(F, S, lay, d, r0, L);
 }
 
 // out = v (accumulate == 0) or out += v
-template <int NC, int V>
-__global__ void __launch_bounds__(RTile<NC, V>::THREADS) k_x_c2r(const float2* __restrict__ S, float* out,
+template <int NC>
+__global__ void __launch_bounds__(RTile<NC, 0>::THREADS) k_x_c2r(const float2* __restrict__ S, float* out,
                                                              int accumulate, Dims d,
                                                              const __grid_constant__ FFTPlan plan,
                                                              const float2* __restrict__ tw_g, int Lrt) {
   extern __shared__ __align__(16) float2 sm[];
   constexpr bool CT = NC > 0;
   const int nx = CT ? NC : d.nx;
-  const int L = row_lines<NC, V>(Lrt);
-  const auto lay = row_lay<NC, V>(nx);
+  const int L = row_lines<NC, 0>(Lrt);
+  const auto lay = row_lay<NC, 0>(nx);
   float2* tw = sm;
   float2* B0 = sm + nx;
-  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, V>(nx);
+  float2* B1 = CT ? nullptr : B0 + L * row_stride<NC, 0>(nx);
   for (int i = threadIdx.x; i < nx; i += blockDim.x) tw[i] = tw_g[i];
   const long long r0 = d.row0 + (long long)blockIdx.x * 2 * L;
   load_c2r<NC>(S, B0, lay, d, r0, L);
   __syncthreads();
-  float2* G = row_fft<NC, V, true>(B0, B1, tw, plan, L, lay);
+  float2* G = row_fft<NC, 0, true>(B0, B1, tw, plan, L, lay);
   const int total = 2 * L * nx;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int q = i / nx, x = i - q * nx;
@@ -1439,22 +1439,22 @@ static void x_eos_t(const EosArgs& a, const Dims& d, const FFTPlan& plan, const 
   launch_pdl(k_x_eos<NC, V>, dim3(row_tiles(d, L)), dim3(RTile<NC, V>::THREADS), sm, st, a, d, plan, tw, L);
 }
 
-template <int NC, int V>
+template <int NC>
 static void x_r2c_t(const float* f, float2* S, const Dims& d, const FFTPlan& plan, const float2* tw, int Lrt,
                     cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
-  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 1 : 2);
-  set_smem(k_x_r2c<NC, V>, sm);
-  k_x_r2c<NC, V><<<row_tiles(d, L), RTile<NC, V>::THREADS, sm, st>>>(f, S, d, plan, tw, L);
+  const int L = NC > 0 ? RTile<NC, 0>::LINES : Lrt;
+  const size_t sm = smem_row<NC, 0>(d.nx, L, NC > 0 ? 1 : 2);
+  set_smem(k_x_r2c<NC>, sm);
+  k_x_r2c<NC><<<row_tiles(d, L), RTile<NC, 0>::THREADS, sm, st>>>(f, S, d, plan, tw, L);
 }
 
-template <int NC, int V>
+template <int NC>
 static void x_c2r_t(const float2* S, float* out, int acc, const Dims& d, const FFTPlan& plan, const float2* tw,
                     int Lrt, cudaStream_t st) {
-  const int L = NC > 0 ? RTile<NC, V>::LINES : Lrt;
-  const size_t sm = smem_row<NC, V>(d.nx, L, NC > 0 ? 1 : 2);
-  set_smem(k_x_c2r<NC, V>, sm);
-  k_x_c2r<NC, V><<<row_tiles(d, L), RTile<NC, V>::THREADS, sm, st>>>(S, out, acc, d, plan, tw, L);
+  const int L = NC > 0 ? RTile<NC, 0>::LINES : Lrt;
+  const size_t sm = smem_row<NC, 0>(d.nx, L, NC > 0 ? 1 : 2);
+  set_smem(k_x_c2r<NC>, sm);
+  k_x_c2r<NC><<<row_tiles(d, L), RTile<NC, 0>::THREADS, sm, st>>>(S, out, acc, d, plan, tw, L);
 }
 
 // The launchers of one length.  Member functions are defined out of class
@@ -1514,12 +1514,12 @@ void CtKernels<NC>::x_eos(const EosArgs& a, const Dims& d, const FFTPlan& plan, 
 template <int NC>
 void CtKernels<NC>::x_r2c(const float* f, float2* S, const Dims& d, const FFTPlan& plan, const float2* tw,
                           int L, cudaStream_t st) {
-  x_r2c_t<NC, 0>(f, S, d, plan, tw, L, st);
+  x_r2c_t<NC>(f, S, d, plan, tw, L, st);
 }
 template <int NC>
 void CtKernels<NC>::x_c2r(const float2* S, float* out, int acc, const Dims& d, const FFTPlan& plan,
                           const float2* tw, int L, cudaStream_t st) {
-  x_c2r_t<NC, 0>(S, out, acc, d, plan, tw, L, st);
+  x_c2r_t<NC>(S, out, acc, d, plan, tw, L, st);
 }
 
 }  // namespace kwb

@@ -35,7 +35,6 @@ struct ColTmaArgs {
 
 struct FusedTmaArgs {
   CUtensorMap in[3];
-  CUtensorMap out[9];
   SpecOp op[9];
   float2* outp[9];      // output buffers (written with plain stores)
   float2* dual_outp[9];         // optional second output: outp times dual_tab[outer]

@@ -934,7 +934,6 @@ void Session::fused_pass(const std::vector<int>& ins, const std::vector<int>& ou
     const CUtensorMap* maps = (d.dim == 3) ? map_z : map_y;
     for (int i = 0; i < nin; ++i) fa.in[i] = maps[ins[i]];
     for (int i = 0; i < nout; ++i) {
-      fa.out[i] = maps[outs[i]];
       fa.outp[i] = Sp(outs[i]);
       fa.op[i] = ops[i];
       if (i < (int)dual.size() && dual[i] >= 0) {
@@ -1368,22 +1367,17 @@ bool Session::graphable(uint64_t t) const {
   return true;
 }
 
-// `steps` steps from t captured as one graph.
-void Session::capture(uint64_t t, int steps, cudaGraph_t* g) {
-  ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-  const uint64_t l0 = launches_;
-  for (int i = 0; i < steps; ++i) enqueue_step_body(t + i);
-  graph_launches = (launches_ - l0) / steps;
-  launches_ = l0;
-  ck(cudaStreamEndCapture(st, g), "end capture");
-}
-
 void Session::enqueue_step() {
   const uint64_t t = t_done + 1;
   if (graphable(t)) {
     if (!graph_exec) {
       cudaGraph_t g = nullptr;
-      capture(t, 1, &g);
+      ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
+      const uint64_t l0 = launches_;
+      enqueue_step_body(t);
+      graph_launches = launches_ - l0;
+      launches_ = l0;
+      ck(cudaStreamEndCapture(st, &g), "end capture");
       graph = g;
       ++graph_gen;
       ck(cudaGraphInstantiate(&graph_exec, graph, 0), "graph instantiate");

@@ -143,7 +143,6 @@ class Session {
   bool use_graph = true;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
-  void capture(uint64_t t, int steps, cudaGraph_t* g);
   void drop_graphs();
   uint64_t graph_launches = 0;
   uint64_t graph_gen = 0;  // captures so far (a batch rebuilds its parent graph when this changes)
