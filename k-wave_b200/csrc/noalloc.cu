@@ -17,8 +17,8 @@
 // its address on the current device with cudaGetSymbolAddress and raises the
 // kernel's shared-memory limit (cheap once the module is loaded, and never
 // stale: a device reset or a new primary context gives a new address).  The
-// first call on a device may load this module onto it, so make that first
-// call, e.g. on a small grid, before any stream capture begins.
+// first call on a device may load this module onto it.  A call on a capturing
+// stream is refused: asking for the stream's device is not permitted then.
 // Twiddle factors and operator values are generated inside the kernel, so
 // nothing is copied from the host either.
 //
@@ -52,9 +52,10 @@ constexpr size_t MAX_SMEM = sizeof(float2) * ((size_t)MAX_EDGE + 3ull * MAX_EDGE
 
 // Columns per CTA in the y pass: the most that still give MIN_COL_BLOCKS CTAs.
 // The spectra (at most 4 MiB each) stay in L2, so the narrow rows of a small
-// tile cost no DRAM traffic, and a call is a chain of latencies: at 384 x 320
-// eight columns meant 25 CTAs with three transforms of 2560 elements one after
-// the other, 34 us of the call's 51.
+// tile cost no DRAM traffic, and a call is a chain of latencies: at 384 x 320,
+// the one grid this was set on, eight columns meant 25 CTAs with three
+// transforms of 2560 elements one after the other (the call took 34.8 us, 22.5
+// with one column per CTA, the light radices and the overlapped launches).
 int col_tile(int nxh) {
   int tl = MAX_TL;
   while (tl > 1 && (nxh + tl - 1) / tl < MIN_COL_BLOCKS) tl /= 2;
