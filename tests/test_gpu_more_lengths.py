@@ -1,7 +1,7 @@
 """Compile-time and TMA-fed kernels of the lengths with a factor 7, from 40 to
 63, and above 256 (whose line one tensor copy covers as several segments).
 
-Against the FP64 oracle at the suite's 1e-4 bar, and the TMA-fed y pass bit for
+Against the FP64 oracle (runs this short meet it at 1e-6; the bar is 1e-5), and the TMA-fed y pass bit for
 bit against the plain column kernel (both run the same radix plan)."""
 import os
 
@@ -31,7 +31,7 @@ def test_against_the_oracle(n):
     inp, record, start, _ = case_3d_het(n=n, nt=8, record=RECORD)
     gpu = _lib.solve(inp, record=record, start_index=start)
     errs = compare(gpu, oracle_outputs(inp, record, start, dtype=np.float64))
-    bad = {k: v for k, v in errs.items() if not v <= 1e-4}
+    bad = {k: v for k, v in errs.items() if not v <= 1e-5}
     assert errs and not bad, errs
 
 
