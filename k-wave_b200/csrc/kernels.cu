@@ -210,6 +210,8 @@ bool ct_supported(int n) { return kernels_for(n).n == n && n > 0; }
 // lossless (0.5 k threads a row pass) 25 / 51, 64 x 72 x 80 absorbing (12 k)
 // 96 / 129; of the x axis alone 1024 x 768 (25 k) 100 / 88, 128^3 (66 k)
 // 177 / 152.
+// No grid between 12 k and 25 k was timed, and a pass of few blocks with many
+// threads each counts as filling the device.
 constexpr long long kNarrowThreads = 148 * 160;
 int plan_variant(int n, long long lines) {
   if (!ct_supported(n)) return 0;
