@@ -99,32 +99,35 @@ __host__ __device__ constexpr CtCost ct_passes(const CtPlan& p) {
 // threads evenly, 12 % where a thread holds over 16 elements, which costs
 // occupancy) or in all (variant 1: latency, with 150 for a pass' barriers and
 // shared-memory round trip and 60 per element for the work around the
-// transform), times 1000.  Runs of whole cases with the overhead of a pass, the
-// held elements' share and the threads varied moved them by up to 20 %: 180 x 150
-// x 125 Stokes, 100 steps, 31.2 to 37.5 ms (125 as 5 x 5 x 5 on 25 or 9 threads),
-// 432 x 360 x 288, 24 steps, 104.7 to 113.8 ms (432 on 48 or 27 threads).
+// transform; up to 80 % more where threads have no butterfly in a pass), times
+// 1000.  Runs of whole cases with the overhead of a pass, the held elements'
+// share and the threads varied moved them by up to 20 %: 180 x 150 x 125 Stokes,
+// 100 steps, 31.2 to 37.5 ms (125 as 5 x 5 x 5 on 25 or 9 threads), 432 x 360 x
+// 288, 24 steps, 104.7 to 113.8 ms (432 on 48 or 27 threads).  Variant 1, us per
+// 2D lossless step with a thread per butterfly of the widest pass or of any:
+// 42 x 256 51 / 37, 1000 x 500 58 / 56, but 256 x 256 27 / 35, 64^3 69 / 82,
+// where most threads then idle.
 __host__ __device__ constexpr long long ct_plan_cost(int n, const CtCost& c, int t, int variant) {
   long long sum = 0;
-  int held = 0;
+  int held = 0, busy = 0;  // busy: thousandths of the threads, summed over the passes
   for (int i = 0; i < c.np; ++i) {
     const int nr = n / c.radix[i], nb = (nr + t - 1) / t;
+    busy += 1000 * nr / (nb * t);
     held = nb * c.radix[i] > held ? nb * c.radix[i] : held;
     sum += variant ? nb * c.work[i] + 150 : nb * c.work[i] * (nr % t ? 11 : 10) + 150;
   }
   if (held > kCtMaxHeld) return -1;
-  if (variant) return 1000 * sum + 60000 * n / t;
+  if (variant) return (sum + 60 * n / t) * (1800 - 800 * busy / (1000 * c.np));
   return sum * t * (held > 16 ? 112 : 100) / n;
 }
 
 __host__ __device__ constexpr void ct_rate(int n, CtPlan& p, CtPlan& best, long long& cost, int variant) {
   const CtCost c = ct_passes(p);
   if (c.np < 2) return;
-  int rmax = 1;
-  for (int i = 0; i < c.np; ++i) rmax = c.radix[i] > rmax ? c.radix[i] : rmax;
-  // threads per line: one butterfly each of the widest pass (variant 1), or 1
-  // to 4 of any pass
-  for (int i = 0; i < (variant ? 1 : 4 * c.np); ++i) {
-    const int nr = n / (variant ? rmax : c.radix[i / 4]), nb = variant ? 1 : i % 4 + 1;
+  // threads per line: one butterfly each of any pass (variant 1), or 1 to 4
+  const int most = variant ? 1 : 4;
+  for (int i = 0; i < most * c.np; ++i) {
+    const int nr = n / c.radix[i / most], nb = i % most + 1;
     const int t = (nr + nb - 1) / nb;
     if (t > 256) continue;
     const long long v = ct_plan_cost(n, c, t, variant);

@@ -205,14 +205,15 @@ const CtEntry& kernels_for(int n, int v = 0) {
 bool ct_supported(int n) { return kernels_for(n).n == n && n > 0; }
 
 // The radix-plan variant (fft_ct.cuh) of `lines` transforms of length n per
-// pass: 1 where variant 0 would leave most of the device idle (fewer than 160
-// threads per SM).  us per step, variants 1 / 0 of every axis: 128 x 128
-// lossless (0.5 k threads a row pass) 25 / 51, 64 x 72 x 80 absorbing (12 k)
-// 96 / 129; of the x axis alone 1024 x 768 (25 k) 100 / 88, 128^3 (66 k)
-// 177 / 152.
-// No grid between 12 k and 25 k was timed, and a pass of few blocks with many
-// threads each counts as filling the device.
-constexpr long long kNarrowThreads = 148 * 160;
+// pass: 1 where variant 0 would leave most of the device idle (fewer than 240
+// threads per SM, 35 520 in all).  us per step, variants 1 / 0 of every axis, at
+// the threads a row pass of variant 0 has: 2D lossless 256^2 (2 k) 27 / 50, 768^2
+// (18 k) 58 / 74, 1024 x 768 (25 k) 72 / 81, 900^2 (27 k) 89 / 96, 960^2 (31 k)
+// 97 / 99, 800^2 (32 k) 72 / 72, 980^2 (34 k) 87 / 105, 1008^2 (36 k) 109 / 90; 3D
+// lossless 64^3 (8 k) 48 / 76, 84^3 (21 k) 89 / 141, 100^3 (25 k) 127 / 129, 98^3
+// (34 k) 138 / 159, 96^3 (37 k) 111 / 105, 90^3 (40 k) 138 / 115, 128^3 (66 k)
+// 190 / 154.
+constexpr long long kNarrowThreads = 148 * 240;
 int plan_variant(int n, long long lines) {
   if (!ct_supported(n)) return 0;
   return lines * kernels_for(n).threads_per_line() < kNarrowThreads ? 1 : 0;
