@@ -29,7 +29,7 @@ namespace kwb {
 // The grouping of a length is found by exhaustive search with the cost model
 // below.  Variant 1 is for grids too small to fill the device, where a step is
 // a chain of latencies: the model then counts one thread's own work, so more
-// threads share a line (128 = 16 x 8 as 4, 4, 4, 2 on 32 threads instead of 8).
+// threads share a line (128 = 16 x 8 as 4, 4, 8 on 32 threads instead of 8).
 // ---------------------------------------------------------------------------
 constexpr int kCtMaxSteps = 16;
 struct CtStep {
